@@ -204,7 +204,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p) {
       if (use > 0)
         tc::mbar_wait(bar_empty + 8 * xs, uint32_t(use - 1) & 1u, abort_flag, &g_gemm_status,
                       tc::kStatusWaitEmpty);
-      if (lane == 0 && !*abort_flag) {
+      if (tc::elect_one() && !*abort_flag) {
         tc::mbar_expect_tx(bar_xfull + 8 * xs, stage_bytes);
         tma_load_2d(xaddr[xs], &xmap, bar_xfull + 8 * xs, c * kChunkK, m0);
       }
@@ -230,7 +230,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p) {
       tc::mbar_wait(bar_xfull + 8 * stage, phase, abort_flag, &g_gemm_status, tc::kStatusWaitLoad);
       tc::mbar_wait(bar_afull + 8 * stage, phase, abort_flag, &g_gemm_status, tc::kStatusWaitFull);
       tc::fence_after_sync();
-      if (lane == 0) {
+      if (tc::elect_one()) {
         const uint32_t a0 = tmem + kACol + 32u * uint32_t(stage), d0 = pass ? dcol[1] : dcol[0];
         tc::mma_ts(d0, a0, bdesc0, idesc, first ? 0u : 1u);   // first k-block of a plane overwrites
         tc::mma_ts(d0, a0 + 8u, bdesc0 + 2u, idesc, 1u);      // +32 bytes of K per step
@@ -785,7 +785,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap xmap,
         if (i >= NS)
           tc::mbar_wait(bar_done + 8 * xs, uint32_t(i / NS - 1) & 1u, abort_flag,
                         &g_gemm_status, tc::kStatusWaitEmpty, p.wait_cycles);
-        if (lane == 0 && !*abort_flag) {
+        if (tc::elect_one() && !*abort_flag) {
           if constexpr (PAIR) {
             // both halves report their bytes to the leader's barrier; the leader expects them
             if (crank == 0) tc::mbar_expect_tx(bar_full + 8 * xs, 2u * stage_bytes);
@@ -809,7 +809,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap xmap,
 #pragma unroll
     for (int s = 0; s < NS; ++s) xlo[s] = uint32_t(dtemplate) + (xstage(s) >> 4);
     const uint32_t xhi = uint32_t(dtemplate >> 32);
-    if (lane == 0 && crank == 0) {               // of a pair only the leader issues
+    if (crank == 0 && tc::elect_one()) {         // of a pair only the leader issues
       int t = -1, c = 0, c_first = 0, c_end = 0;   // segment, k-block, the segment's k range
       uint32_t idesc = 0;
       const uint32_t d0 = tmem;
