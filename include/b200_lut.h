@@ -487,6 +487,12 @@ int b200lut_embed_gather(const int64_t* ids, int64_t n_ids, int K, int dtype,
                          const b200lut_segment* table, const void* resB, int out_fp32,
                          void* stream);
 
+/* The same, and *bad_id (device, may be NULL) is set to 1 when an id was out of range: a caller's
+ * own record, which other tables' gathers do not touch. It is never cleared here. */
+int b200lut_embed_gather_checked(const int64_t* ids, int64_t n_ids, int K, int dtype,
+                                 const b200lut_segment* table, const void* resB, int out_fp32,
+                                 int32_t* bad_id, void* stream);
+
 /* out[m, k] = round_to_dtype(in[m, k]) for fp32 rows (the `.to(lut.dtype)` that ends the
  * reference's embedding forward, :2335). */
 int b200lut_round_rows(const float* in, int64_t ldi, void* out, int64_t ldo, int64_t M, int K,

@@ -8,6 +8,7 @@ stream so they order with the surrounding torch work.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 from typing import Optional, Sequence
 
@@ -32,7 +33,7 @@ EXPORTS = (
     "b200lut_gemv_multi", "b200lut_gemv", "b200lut_gemm", "b200lut_fht",
     "b200lut_residual_project", "b200lut_residual_project_rows", "b200lut_silu_mul", "b200lut_gemm_workspace_bytes", "b200lut_gemm_ws", "b200lut_gemm_multi",
     "b200lut_gemm_two_stream", "b200lut_gemm_two_stream_bytes",
-    "b200lut_embed_gather", "b200lut_round_rows", "b200lut_gemv_kgrouped",
+    "b200lut_embed_gather", "b200lut_embed_gather_checked", "b200lut_round_rows", "b200lut_gemv_kgrouped",
     "b200lut_gemv_kgrouped_split", "b200lut_gemv_kgrouped_workspace_bytes", "b200lut_gemm_kgrouped", "b200lut_gemv_exchange", "b200lut_peer_export", "b200lut_peer_open", "b200lut_peer_close",
     "b200lut_gemv_noalloc", "b200lut_gemv_noalloc_reset", "b200lut_gemv_launch_blocks", "b200lut_gemv_input", "b200lut_plan_bytes", "b200lut_plan_build", "b200lut_plan_run", "b200lut_plan_status", "b200lut_plan_form", "b200lut_plan_release",
 )
@@ -143,6 +144,8 @@ def lib() -> ctypes.CDLL:
     L.b200lut_gemm_two_stream.argtypes = [vp, i64, i32, i32, i32, ctypes.POINTER(Segment), i32, vp, sz, vp]
     L.b200lut_embed_gather.restype = i32
     L.b200lut_embed_gather.argtypes = [vp, i64, i32, i32, ctypes.POINTER(Segment), vp, i32, vp]
+    L.b200lut_embed_gather_checked.restype = i32
+    L.b200lut_embed_gather_checked.argtypes = [vp, i64, i32, i32, ctypes.POINTER(Segment), vp, i32, vp, vp]
     L.b200lut_round_rows.restype = i32
     L.b200lut_round_rows.argtypes = [vp, i64, vp, i64, i64, i32, i32, vp]
     L.b200lut_silu_mul.restype = i32
@@ -191,6 +194,30 @@ def lib() -> ctypes.CDLL:
     return L
 
 
+HOST_PATH = os.path.join(_HERE, "_b200lut_host.so")
+
+
+class _Host:
+    """The native host layer (extension module _b200lut_host, built next to the library), loaded on
+    first use; from then on its functions are plain attributes of this object."""
+
+    def __getattr__(self, name):
+        if name.startswith("__"):
+            raise AttributeError(name)
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python {os.path.join(_HERE, 'build.py')}`")
+        spec = importlib.util.spec_from_file_location("_b200lut_host", HOST_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.set_library_error(LibraryError)
+        self.__dict__.update({k: getattr(mod, k) for k in dir(mod) if not k.startswith("__")})
+        return getattr(mod, name)
+
+
+host = _Host()
+
+
 def check(code: int) -> None:
     if code != OK:
         raise LibraryError(code, lib().b200lut_last_error().decode("utf-8", "replace"))
@@ -207,7 +234,26 @@ def dtype_id(dtype: torch.dtype) -> int:
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
+
+
+class _NoGuard:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return None
+
+
+_NO_GUARD = _NoGuard()
+
+
+def _on_device(device: torch.device):
+    """Device guard that costs nothing when `device` is current already."""
+    index = device.index
+    if index is None or index == torch._C._cuda_getDevice():
+        return _NO_GUARD
+    return torch.cuda.device(device)
 
 
 def _need_cuda(t: torch.Tensor, what: str) -> None:
@@ -306,7 +352,7 @@ def residual_project(x: torch.Tensor, resB: torch.Tensor, flags: int = 0,
     R = resB.shape[0]
     if out is None:
         out = torch.empty(M, R, dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         check(lib().b200lut_residual_project(x.data_ptr(), x.stride(0), M, K, dtype_id(x.dtype),
                                              resB.data_ptr(), R, out.data_ptr(), out.stride(0),
                                              flags, _stream(x)))
@@ -330,7 +376,7 @@ def residual_project_rows(x: torch.Tensor, resB: torch.Tensor, flags: int = 0,
         out = torch.empty(M, cols, dtype=x.dtype, device=x.device)
     if out.shape[1] != cols or out.dtype != x.dtype or out.stride(1) != 1:
         raise ValueError("residual_project_rows: out must be [M, 64 * ceil(R / 64)] in x's dtype")
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         check(lib().b200lut_residual_project_rows(x.data_ptr(), x.stride(0), M, K, dtype_id(x.dtype),
                                                   resB.data_ptr(), R, out.data_ptr(), out.stride(0),
                                                   cols, flags, _stream(x)))
@@ -349,7 +395,7 @@ def gemv_multi(x: torch.Tensor, segs, nseg: int, epilogue: int = EPI_NONE, split
     M, K = x.shape
     ws_ptr = None if workspace is None else workspace.data_ptr()
     ws_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         check(lib().b200lut_gemv_multi(x.data_ptr(), x.stride(0), M, K, dtype_id(x.dtype), segs,
                                        nseg, epilogue, split, ws_ptr, ws_bytes, flags, _stream(x)))
 
@@ -371,7 +417,7 @@ def gemv_exchange(x: torch.Tensor, segs, nseg: int, ex: "Exchange", epilogue: in
     """gemv_multi with the column-parallel exchange folded in (push after, wait before)."""
     _need_cuda(x, "x")
     M, K = x.shape
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         check(lib().b200lut_gemv_exchange(x.data_ptr(), x.stride(0), M, K, dtype_id(x.dtype), segs,
                                           nseg, epilogue, split, None, 0, flags,
                                           ctypes.byref(ex), _stream(x)))
@@ -407,7 +453,7 @@ def gemv_input(x: torch.Tensor, segs, nseg: int, inp: Input, epilogue: int = EPI
     rotation); raises LibraryError (code 2) when the shapes are not served in fused form."""
     _need_cuda(x, "x")
     M, K = x.shape
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         check(lib().b200lut_gemv_input(x.data_ptr(), x.stride(0), M, K, dtype_id(x.dtype), segs, nseg,
                                        epilogue, 0, None, 0, flags,
                                        None if ex is None else ctypes.byref(ex), ctypes.byref(inp), _stream(x)))
@@ -437,18 +483,20 @@ def silu_mul(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     """gate <- silu(gate) * up, in place (2-D, last dim contiguous, 16-bit)."""
     _need_cuda(gate, "gate")
     M, N = gate.shape
-    with torch.cuda.device(gate.device):
+    with _on_device(gate.device):
         check(lib().b200lut_silu_mul(gate.data_ptr(), up.data_ptr(), M, N, gate.stride(0), up.stride(0),
                                      dtype_id(gate.dtype), _stream(gate)))
     return gate
 
 
 def embed_gather(ids: torch.Tensor, table: dict, K: int, dtype: torch.dtype,
-                 out_fp32: bool = False, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                 out_fp32: bool = False, out: Optional[torch.Tensor] = None,
+                 bad: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Rows ids (1-D int64 CUDA tensor) of a palettized [N, K] table -> [n, K] in `dtype`
     (fp32 with out_fp32). table: packed, lut, bits, N, group_size, n_groups and optionally
     packed2 / lut2 / bits2 and resA + resB (both or neither). out: a contiguous [n, K] tensor of
-    the result type to write into (nothing is allocated then)."""
+    the result type to write into (nothing is allocated then). bad: an int32 CUDA tensor [1] that is
+    set to 1 when an id is out of range."""
     _need_cuda(ids, "ids")
     if ids.dim() != 1 or ids.dtype != torch.int64 or not ids.is_contiguous():
         raise ValueError("embed_gather expects a contiguous 1-D int64 id tensor")
@@ -469,9 +517,9 @@ def embed_gather(ids: torch.Tensor, table: dict, K: int, dtype: torch.dtype,
     resA, resB = table.get("resA"), table.get("resB")
     if resA is not None:
         s.resA, s.res_rank = ptr(resA), int(resA.shape[1])
-    with torch.cuda.device(ids.device):
-        check(lib().b200lut_embed_gather(ids.data_ptr(), n, K, dtype_id(dtype), seg, ptr(resB),
-                                         1 if out_fp32 else 0, _stream(ids)))
+    with _on_device(ids.device):
+        check(lib().b200lut_embed_gather_checked(ids.data_ptr(), n, K, dtype_id(dtype), seg, ptr(resB),
+                                                 1 if out_fp32 else 0, ptr(bad), _stream(ids)))
     return out
 
 
@@ -480,7 +528,7 @@ def round_rows(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     _need_cuda(x, "x")
     M, K = x.shape
     out = torch.empty(M, K, dtype=dtype, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         check(lib().b200lut_round_rows(x.data_ptr(), x.stride(0), out.data_ptr(), K, M, K,
                                        dtype_id(dtype), _stream(x)))
     return out
@@ -489,17 +537,11 @@ def round_rows(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
 _gemm_scratch = {}
 
 
-def _gemm_workspace(device: torch.device, stream: int, nbytes: int) -> torch.Tensor:
-    """Scratch of the prefill GEMM's split schedule, one per device and stream (a buffer serves
-    one launch at a time, and launches of one stream are ordered): zero-filled when
-    (re)allocated, grown geometrically."""
-    key = (device, stream)
-    buf = _gemm_scratch.get(key)
-    if buf is None or buf.numel() < nbytes:
-        size = max(nbytes, 2 * buf.numel() if buf is not None else 0)
-        buf = torch.zeros(size, dtype=torch.uint8, device=device)
-        _gemm_scratch[key] = buf
-    return buf
+def _gemm_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
+    """Scratch of the prefill GEMM's split schedule for the current stream (a buffer serves one
+    launch at a time, and launches of one stream are ordered): zero-filled when (re)allocated,
+    grown geometrically, a graph capture has its own (csrc/host/scratch.h)."""
+    return host.workspace(device.index if device.index is not None else torch.cuda.current_device(), nbytes)
 
 
 def gemm(x: torch.Tensor, seg, epilogue: int = EPI_NONE, flags: int = 0, split: bool = True) -> None:
@@ -507,11 +549,11 @@ def gemm(x: torch.Tensor, seg, epilogue: int = EPI_NONE, flags: int = 0, split: 
     shape gains from it (split=False: whole-tile schedule)."""
     _need_cuda(x, "x")
     M, K = x.shape
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         s0 = seg[0]
         need = lib().b200lut_gemm_workspace_bytes(M, int(s0.N), K) if (split and not s0.packed2) else 0
         if need:
-            ws = _gemm_workspace(x.device, int(_stream(x) or 0), need)
+            ws = _gemm_workspace(x.device, need)
             check(lib().b200lut_gemm_ws(x.data_ptr(), x.stride(0), M, K, dtype_id(x.dtype), seg,
                                         epilogue, flags, ws.data_ptr(), ws.numel(), _stream(x)))
         else:
@@ -531,7 +573,7 @@ def gemv_kgrouped(x: torch.Tensor, packed: torch.Tensor, lut_k: torch.Tensor, N:
     M, K = x.shape
     if out is None:
         out = torch.empty(M, N, dtype=x.dtype, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         # split = 0 leaves the choice (kernel and split) to the library; the scratch is sized for
         # the split it would pick for its workspace-folded kernel
         planned = split if split > 0 else lib().b200lut_gemv_kgrouped_split(N, K)
@@ -565,9 +607,9 @@ def gemm_kgrouped(x: torch.Tensor, packed: torch.Tensor, lut_k: torch.Tensor, N:
     M, K = x.shape
     if out is None:
         out = torch.empty(M, N, dtype=x.dtype, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         need = lib().b200lut_gemm_workspace_bytes(M, N, K) if split else 0
-        ws = _gemm_workspace(x.device, int(_stream(x) or 0), need) if need else None
+        ws = _gemm_workspace(x.device, need) if need else None
         check(lib().b200lut_gemm_kgrouped(x.data_ptr(), x.stride(0), M, K, dtype_id(x.dtype),
                                           packed.data_ptr(), lut_k.data_ptr(), ptr(bias), N, bits,
                                           out.data_ptr(), out.stride(0), flags, ptr(ws),
@@ -580,7 +622,7 @@ def gemm_two_stream(x: torch.Tensor, seg, flags: int = 0) -> None:
     launches that share fp32 sums through a scratch buffer, one rounding."""
     _need_cuda(x, "x")
     M, K = x.shape
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         need = lib().b200lut_gemm_two_stream_bytes(M, int(seg[0].N))
         key = (x.device, int(_stream(x) or 0), "two")
         buf = _gemm_scratch.get(key)
@@ -610,10 +652,10 @@ def gemm_multi(x: torch.Tensor, segs, nseg: int, flags: int = 0, split: bool = T
     """Prefill GEMM over `nseg` projections that share x, as one launch."""
     _need_cuda(x, "x")
     M, K = x.shape
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         total = sum(int(segs[i].N) for i in range(nseg))
         need = lib().b200lut_gemm_workspace_bytes(M, total, K) if split else 0
-        ws = _gemm_workspace(x.device, int(_stream(x) or 0), need) if need else None
+        ws = _gemm_workspace(x.device, need) if need else None
         check(lib().b200lut_gemm_multi(x.data_ptr(), x.stride(0), M, K, dtype_id(x.dtype), segs, nseg,
                                        flags, ptr(ws), ws.numel() if ws is not None else 0, _stream(x)))
 
@@ -632,7 +674,7 @@ def fht(x: torch.Tensor, signs: Optional[torch.Tensor], mode: int = FHT_FORWARD,
         if v is not None and (v.dtype != torch.float32 or not v.is_contiguous()
                               or v.numel() != K or v.device != x.device):
             raise ValueError(f"{name} must be a contiguous (K,) float32 tensor on x's device")
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         check(lib().b200lut_fht(x.data_ptr(), out.data_ptr(), ptr(signs), ptr(scale), M, K,
                                 x.stride(0), out.stride(0), dtype_id(x.dtype), mode, block,
                                 _stream(x)))

@@ -47,7 +47,14 @@ struct EmbedParams {
   int out_f32;
   int vec_ok;             // 16-byte stores allowed
   int N, K, group_size, n_groups;
+  int* bad;               // the caller's own record of an out-of-range id, or null
 };
+
+// An id outside the table: recorded for the library's status word and for the caller.
+__device__ __forceinline__ void record_bad_id(const EmbedParams& p) {
+  atomicExch(&g_embed_status, kBadId);
+  if (p.bad) atomicExch(p.bad, 1);
+}
 
 // the 8 codes k0 .. k0+7 (k0 % 8 == 0) of tile row r in the chunk at `chunk`
 __device__ __forceinline__ void row_codes8(const uint8_t* chunk, int r, int kk0, int bits,
@@ -87,7 +94,7 @@ __global__ void __launch_bounds__(kEmbedThreads) embed_gather_kernel(const Embed
 #pragma unroll
   for (int e = 0; e < 8; ++e) v[e] = 0.f;
   if (id < 0 || id >= p.N) {
-    if (threadIdx.x == 0 && blockIdx.y == 0) atomicExch(&g_embed_status, kBadId);
+    if (threadIdx.x == 0 && blockIdx.y == 0) record_bad_id(p);
   } else {
     const int n = int(id), t = n >> 7, r = n & 127;
     int grp = n / p.group_size;
@@ -169,7 +176,7 @@ __global__ void __launch_bounds__(kEmbedThreads) embed_gather4_kernel(const Embe
   uint16_t* orow = static_cast<uint16_t*>(p.out) + tok * p.ldo;
   const int G = p.K / kChunkK;
   if (id < 0 || id >= p.N) {
-    if (threadIdx.x == 0) atomicExch(&g_embed_status, kBadId);
+    if (threadIdx.x == 0) record_bad_id(p);
     for (int item = threadIdx.x; item < G * 16; item += kEmbedThreads)
       *reinterpret_cast<uint2*>(orow + item * 4) = make_uint2(0u, 0u);
     return;
@@ -221,6 +228,12 @@ using namespace b200lut;
 extern "C" int b200lut_embed_gather(const int64_t* ids, int64_t n_ids, int K, int dtype,
                                     const b200lut_segment* table, const void* resB, int out_fp32,
                                     void* stream) {
+  return b200lut_embed_gather_checked(ids, n_ids, K, dtype, table, resB, out_fp32, nullptr, stream);
+}
+
+extern "C" int b200lut_embed_gather_checked(const int64_t* ids, int64_t n_ids, int K, int dtype,
+                                            const b200lut_segment* table, const void* resB,
+                                            int out_fp32, int32_t* bad_id, void* stream) {
   B200LUT_REQUIRE(table, B200LUT_ERR_INVALID, "null table descriptor");
   const b200lut_segment& s = *table;
   B200LUT_REQUIRE(n_ids >= 0 && n_ids <= 0x7fffffffLL, B200LUT_ERR_INVALID,
@@ -245,6 +258,7 @@ extern "C" int b200lut_embed_gather(const int64_t* ids, int64_t n_ids, int K, in
                       (s.res_rank == 0 || aligned16(resB)),
                   B200LUT_ERR_ALIGN, "codes must be 4-byte aligned and resB 16-byte aligned");
   EmbedParams p = {};
+  p.bad = bad_id;
   p.ids = reinterpret_cast<const long long*>(ids);
   p.packed[0] = static_cast<const uint8_t*>(s.packed);
   p.packed[1] = static_cast<const uint8_t*>(s.packed2);

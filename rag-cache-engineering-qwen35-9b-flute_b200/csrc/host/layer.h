@@ -1,0 +1,102 @@
+// Native description of one palettized projection, kept in its module's __dict__ as "_native".
+//
+// The module stays the owner of its state: a description remembers which objects (and which
+// storage) it was built from and is only used while the module still holds exactly those, so
+// .to(), drop_blob(), a replaced palette or a changed option all lead back to the Python route,
+// which builds a new one.
+#pragma once
+
+#include <Python.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <ATen/ATen.h>
+
+#include <cstdint>
+#include <cstdlib>
+#include <vector>
+
+#include "../../../include/b200_lut.h"
+
+namespace b200host {
+
+// One entry of the module that the description depends on.
+struct Watch {
+  PyObject* key;        // interned name
+  PyObject* value;      // the object found under it when the description was built, or null
+  const void* data;     // a tensor's storage address (null for other objects)
+  bool in_params;       // looked up in _parameters instead of _buffers / __dict__
+};
+
+struct Layer {
+  PyObject_HEAD
+  bool ready;
+  int N, K, bits, bits2, group, n_groups, device, dtype;     // dtype: B200LUT_BF16 / B200LUT_F16
+  at::ScalarType scalar;
+  bool two, res, res_ok, rotated, kgrouped;
+  int pow2_segments;
+  PyObject* rotation;                       // key of the fold (equal keys: the same rotation), or null
+  at::Tensor *packed, *lut, *packed2, *lut2, *bias, *resA, *resB, *signs, *awq;
+  std::vector<Watch>* watches;
+};
+
+inline PyObject* name_buffers() { static PyObject* s = PyUnicode_InternFromString("_buffers"); return s; }
+inline PyObject* name_params() { static PyObject* s = PyUnicode_InternFromString("_parameters"); return s; }
+inline PyObject* name_modules() { static PyObject* s = PyUnicode_InternFromString("_modules"); return s; }
+inline PyObject* name_native() { static PyObject* s = PyUnicode_InternFromString("_native"); return s; }
+
+// Where a module keeps `key`: a buffer shadows a plain attribute (both exist for optional tensors).
+inline PyObject* lookup(PyObject* dict, PyObject* key, bool in_params) {
+  PyObject* group = PyDict_GetItemWithError(dict, in_params ? name_params() : name_buffers());
+  if (group && PyDict_Check(group)) {
+    PyObject* v = PyDict_GetItemWithError(group, key);
+    if (v) return v;
+  }
+  return PyDict_GetItemWithError(dict, key);
+}
+
+inline const void* storage_of(PyObject* o) {
+  return o && THPVariable_Check(o) ? THPVariable_Unpack(o).const_data_ptr() : nullptr;
+}
+
+inline bool current(const Layer& l, PyObject* dict) {
+  for (const Watch& w : *l.watches) {
+    PyObject* v = lookup(dict, w.key, w.in_params);
+    if (v != w.value) return false;
+    if (w.data && storage_of(v) != w.data) return false;
+  }
+  return true;
+}
+
+extern PyTypeObject LayerType;
+
+// The module's description if it may be used, else null (never sets an exception).
+inline Layer* layer_of(PyObject* dict) {
+  PyObject* o = PyDict_GetItemWithError(dict, name_native());
+  if (!o || Py_TYPE(o) != &LayerType) return nullptr;
+  Layer* l = reinterpret_cast<Layer*>(o);
+  if (!l->ready) return nullptr;
+  if (!current(*l, dict)) {
+    PyDict_SetItem(dict, name_native(), Py_None);     // the Python route builds a new one
+    return nullptr;
+  }
+  return l;
+}
+
+// Child module `name` of a module's __dict__: its own __dict__ (borrowed), or null.
+inline PyObject* child_dict(PyObject* dict, PyObject* name, PyObject** child = nullptr) {
+  PyObject* mods = PyDict_GetItemWithError(dict, name_modules());
+  PyObject* m = mods && PyDict_Check(mods) ? PyDict_GetItemWithError(mods, name) : nullptr;
+  if (child) *child = m;
+  if (!m) return nullptr;
+  PyObject* d = PyObject_GenericGetDict(m, nullptr);
+  if (!d) { PyErr_Clear(); return nullptr; }
+  Py_DECREF(d);                                       // the object keeps it
+  return d;
+}
+
+inline bool env_on(const char* name) {
+  const char* e = std::getenv(name);
+  return e && (e[0] == '1' || e[0] == 't' || e[0] == 'T');
+}
+
+}  // namespace b200host

@@ -93,6 +93,10 @@ def _vec(v: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
 
 
 def _run(x: torch.Tensor, signs, mode: int, scale=None, block: int = 0, out=None) -> torch.Tensor:
+    if out is None:
+        y = _lib.host.fht(x, signs, scale, mode, block)
+        if y is not None:
+            return y
     K = x.shape[-1]
     x2 = x.reshape(-1, K)
     if x2.stride(-1) != 1:

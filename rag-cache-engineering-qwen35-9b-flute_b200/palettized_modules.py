@@ -253,6 +253,32 @@ class PalettizedLinear(nn.Module):
             raise ValueError("from_packed: wrong code buffer size")
         return mod
 
+    # what the native description is built from: it is used while the module holds these objects
+    _WATCHED = ("lut", "lut2", "resA", "resB", "indices2", "_packed", "_packed2", "N", "K", "bitwidth", "bitwidth2",
+                "group_size", "reference", "rot_signs", "awq_scale", "fold_order", "rotation_seed", "rotation_k")
+
+    def _bind(self) -> None:
+        """Describe the layer to the native host layer (csrc/host), which then serves the forwards that
+        need no conversion; a change of the module's state makes it drop the description."""
+        if self.__dict__.get("_native") is not None or self.reference or not self.lut.is_cuda:
+            return
+        if self.lut.dtype not in (torch.float16, torch.bfloat16) or not self.lut.is_contiguous() or not self.N or not self.K:
+            return
+        if (self.has_stream2 and self.lut2.dtype != self.lut.dtype) or \
+                (self.bias is not None and self.bias.dtype != self.lut.dtype):
+            return
+        self._ensure_packed()
+        spec = dict(packed=self._packed, lut=self.lut, bias=self.bias, resA=self.resA, resB=self.resB, N=self.N, K=self.K,
+                    bits=self.bitwidth, group_size=self.group_size, n_groups=self.lut.shape[0],
+                    watch=self._WATCHED, watch_params=("bias",))
+        if self.has_stream2:
+            spec.update(packed2=self._packed2, lut2=self.lut2, bits2=self.bitwidth2)
+        if self.rot_signs is not None:
+            signs, awq = self._fold(self.lut.device)
+            spec.update(signs=signs, awq=awq, rotation=(self.rotation_seed, self.rotation_k, self.fold_order,
+                                                        None if self.awq_scale is None else id(self.awq_scale)))
+        self.__dict__["_native"] = _lib.host.bind(self.__dict__, spec)
+
     # ---------------------------------------------------------------- pieces
     def _segment_desc(self, out: Optional[torch.Tensor], ldo: Optional[int] = None,
                       with_bias: bool = True, res_t: Optional[torch.Tensor] = None) -> dict:
@@ -427,6 +453,13 @@ class PalettizedLinear(nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if not x.is_cuda:
             raise RuntimeError("PalettizedLinear.forward: x must be a CUDA tensor")
+        out = _lib.host.linear(self.__dict__, x, _LAUNCH_FLAGS["pdl"])
+        if out is None:      # not described yet, or a call that needs conversions
+            out = self._forward_route(x)
+            self._bind()
+        return out
+
+    def _forward_route(self, x: torch.Tensor) -> torch.Tensor:
         shape = x.shape
         if x.shape[-1] != self.K:
             raise ValueError(f"PalettizedLinear: input feature dim {x.shape[-1]} != K {self.K}")
@@ -616,6 +649,12 @@ def _merged_decode(owner: nn.Module, mods, x: torch.Tensor, epilogue: int = None
     return out
 
 
+def _bind_all(mods) -> None:
+    for m in mods:
+        if isinstance(m, PalettizedLinear):
+            m._bind()
+
+
 class SplitQKV(nn.Module):
     """q/k/v projections sharing one input: one merged decode launch when
     M <= 16, else the three modules (reference palettized_modules.py:1390-1466)."""
@@ -625,6 +664,13 @@ class SplitQKV(nn.Module):
         self.q_proj, self.k_proj, self.v_proj = q_proj, k_proj, v_proj
 
     def forward(self, x):
+        out = _lib.host.qkv(self.__dict__, x, _LAUNCH_FLAGS["pdl"])
+        if out is None:
+            out = self._forward_route(x)
+            _bind_all((self.q_proj, self.k_proj, self.v_proj))
+        return out
+
+    def _forward_route(self, x):
         mods = (self.q_proj, self.k_proj, self.v_proj)
         if _prefill_mergeable(mods, x):      # M > 16: one tensor-core launch for the three
             total = sum(m.N for m in mods)
@@ -651,7 +697,10 @@ class FusedPalettizedMLP(nn.Module):
         self.act_fn = act_fn
 
     def _is_silu(self) -> bool:
-        return isinstance(self.act_fn, nn.SiLU) or self.act_fn in (torch.nn.functional.silu,)
+        act = self._modules.get("act_fn")
+        if act is None:
+            act = self.act_fn
+        return isinstance(act, nn.SiLU) or act in (torch.nn.functional.silu,)
 
     def fused_gate_up(self, x2: torch.Tensor) -> torch.Tensor:
         """silu(gate(x2)) * up(x2) for rows already in the projections' basis, one launch."""
@@ -667,6 +716,13 @@ class FusedPalettizedMLP(nn.Module):
         return out
 
     def forward(self, x):
+        out = _lib.host.mlp(self.__dict__, x, _LAUNCH_FLAGS["pdl"]) if self._is_silu() else None
+        if out is None:
+            out = self._forward_route(x)
+            _bind_all((self.gate_proj, self.up_proj, self.down_proj))
+        return out
+
+    def _forward_route(self, x):
         mods = (self.gate_proj, self.up_proj)
         merge = (self._is_silu() and mods[0].N == mods[1].N
                  and os.environ.get("FLUTE_NO_MERGE", "").strip() not in ("1", "true", "True"))
@@ -886,7 +942,40 @@ class PalettizedEmbedding(nn.Module):
                      resB=self.resB.to(self.lut.dtype).contiguous())
         return d
 
+    def _bind(self) -> None:
+        if self.__dict__.get("_native") is not None or self.rot_signs is not None or not self.lut.is_contiguous():
+            return
+        if (self.has_stream2 and self.lut2.dtype != self.lut.dtype) or \
+                (self.has_residual() and (self.resA.dtype != self.lut.dtype or self.resB.dtype != self.lut.dtype)):
+            return
+        t = self._table()
+        spec = dict(packed=t["packed"], lut=self.lut, packed2=t.get("packed2"), lut2=self.lut2, resA=self.resA,
+                    resB=self.resB, N=self.N, K=self.K, bits=self.bitwidth, bits2=self.bitwidth2,
+                    group_size=self.group_size, n_groups=self.lut.shape[0],
+                    watch=("lut", "lut2", "resA", "resB", "indices2", "_packed", "_packed2", "_tied", "N", "K", "bitwidth",
+                           "bitwidth2", "group_size", "rot_signs"))
+        self.__dict__["_native"] = _lib.host.bind(self.__dict__, spec)
+
+    def _bad_id_flag(self) -> torch.Tensor:
+        """Device word that a gather sets when it meets an id outside [0, N)."""
+        flag = self.__dict__.get("_bad_id_word")
+        if flag is None or flag.device != self.lut.device:
+            flag = self.__dict__["_bad_id_word"] = torch.zeros(1, dtype=torch.int32, device=self.lut.device)
+        return flag
+
     def forward(self, ids):
+        native = self.__dict__.get("_native")
+        if native is not None:
+            flag = self._bad_ids if self._bad_ids is not None else self._bad_id_flag()
+            out = _lib.host.embed(self.__dict__, ids, flag)
+            if out is not None:
+                self.__dict__["_bad_ids"] = flag
+                return out
+        out = self._forward_route(ids)
+        self._bind()
+        return out
+
+    def _forward_route(self, ids):
         if not torch.is_tensor(ids):
             ids = torch.as_tensor(ids)
         if ids.dtype not in (torch.int64, torch.int32, torch.int16, torch.int8, torch.uint8):
@@ -897,18 +986,18 @@ class PalettizedEmbedding(nn.Module):
                              f"{int(ids.min())}, max {int(ids.max())}); refusing a silent wrap")
         table = self._table()
         flat = ids.to(device=self.lut.device, dtype=torch.int64).reshape(-1).contiguous()
+        bad = None
         if ids.is_cuda and flat.numel():
             # Device-resident ids cannot be refused here without a host sync (the reference
             # asserts on the device, which would lose the context). The kernel writes zeros for
-            # such an id; the module remembers that it happened, without a sync, and
-            # check_ids() raises at a moment the host chooses.
-            bad = ((flat < 0) | (flat >= self.N)).any()
-            self._bad_ids = bad if self._bad_ids is None else (self._bad_ids | bad)
+            # such an id and sets the module's device word; check_ids() raises at a moment the
+            # host chooses.
+            bad = self.__dict__["_bad_ids"] = self._bad_id_flag()
         dtype = self.lut.dtype
         if self.rot_signs is None:
-            out = _lib.embed_gather(flat, table, self.K, dtype)
+            out = _lib.embed_gather(flat, table, self.K, dtype, bad=bad)
         else:
-            w = _lib.embed_gather(flat, table, self.K, dtype, out_fp32=True)
+            w = _lib.embed_gather(flat, table, self.K, dtype, out_fp32=True, bad=bad)
             if flat.numel():
                 w = _lib.fht(w, self._signs_on(w.device), _lib.FHT_ADJOINT, out=w)
             out = _lib.round_rows(w, dtype)
@@ -921,6 +1010,7 @@ class PalettizedEmbedding(nn.Module):
         status word (0x6000) that the gather kernel raised."""
         bad, self._bad_ids = self._bad_ids, None
         if bad is not None and bool(bad.item()):
+            bad.zero_()
             _lib.lib().b200lut_device_status()
             raise ValueError(f"PalettizedEmbedding: ids out of range [0, {self.N}) were gathered as "
                              f"zero rows since the last check")
@@ -971,7 +1061,24 @@ class KGroupedPalettizedLinear(nn.Module):
         if self._packed is None or self._packed.device != dev:
             self._packed = _lib.repack_from_idxn(self.indices.to(dev), self.N, self.K, self.bitwidth)
 
+    def _bind(self) -> None:
+        if self.__dict__.get("_native") is not None or (self.bias is not None and self.bias.dtype != self.lut_k.dtype):
+            return
+        self._ensure_packed()
+        if self.lut_k.is_contiguous():
+            spec = dict(packed=self._packed, lut=self.lut_k, bias=self.bias, N=self.N, K=self.K, bits=self.bitwidth,
+                        group_size=self.GROUP_K, n_groups=self.N, kgrouped=1,
+                        watch=("lut_k", "_packed", "N", "K", "bitwidth"), watch_params=("bias",))
+            self.__dict__["_native"] = _lib.host.bind(self.__dict__, spec)
+
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        out = _lib.host.kgrouped(self.__dict__, x, _LAUNCH_FLAGS["pdl"])
+        if out is None:
+            out = self._forward_route(x)
+            self._bind()
+        return out
+
+    def _forward_route(self, x: torch.Tensor) -> torch.Tensor:
         if x.shape[-1] != self.K:
             raise ValueError(f"KGroupedPalettizedLinear: input feature dim {x.shape[-1]} != K {self.K}")
         if not x.is_cuda:

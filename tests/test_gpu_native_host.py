@@ -1,0 +1,90 @@
+"""The native host layer (csrc/host) against the Python route it stands in for: the same launches,
+so the same bits, over the row counts where the route changes (decode, tensor-core GEMM) and the
+options it carries; and what makes it let go of a module (replaced palette, swapped bias storage,
+other dtype or device state), where results have to follow the module."""
+from __future__ import annotations
+
+import copy
+
+import pytest
+import torch
+
+from helpers import TOL, Case, pkg, rel_err
+
+pytestmark = pytest.mark.gpu
+
+OPTIONS = (dict(), dict(bias=True, residual=16), dict(rotation_seed=3), dict(rotation_seed=3, residual=8, awq=True),
+           dict(bits2=2, bias=True), dict(bits2=4))
+
+
+@pytest.mark.parametrize("opts", range(len(OPTIONS)))
+@pytest.mark.parametrize("M", (1, 8, 9, 16, 17, 130))
+def test_linear_equals_the_python_route(M, opts):
+    case = Case(256, 192, 64, 4, torch.float16, seed=70 + opts, **OPTIONS[opts])
+    mod = case.module()
+    x = case.x(M).cuda()
+    want = mod._forward_route(x)
+    mod(x)
+    assert mod._native is not None
+    got = pkg._lib.host.linear(mod.__dict__, x, True)
+    if got is not None:                     # None: this row count needs the Python route
+        assert torch.equal(got, want)
+    assert torch.equal(mod(x.view(1, M, 192)).view(M, -1), want)
+    assert rel_err(want, case.oracle(case.x(M))) <= TOL
+
+
+@pytest.mark.parametrize("M", (1, 8, 16, 40))
+@pytest.mark.parametrize("opts", (0, 1, 2))
+def test_merged_modules_equal_the_python_route(M, opts):
+    K = 256
+    mk = lambda n, k, s: Case(n, k, 128, 4, torch.bfloat16, seed=s, **OPTIONS[opts]).module()     # noqa: E731
+    qkv = pkg.SplitQKV(mk(256, K, 1), mk(128, K, 2), mk(128, K, 3))
+    mlp = pkg.FusedPalettizedMLP(mk(384, K, 4), mk(384, K, 5), mk(K, 384, 6), torch.nn.SiLU())
+    x = torch.randn(M, K, device="cuda").bfloat16()
+    for mod in (qkv, mlp):
+        want = mod._forward_route(x)
+        mod(x)
+        assert torch.equal(mod(x), want)
+        host = pkg._lib.host.qkv if mod is qkv else pkg._lib.host.mlp
+        assert torch.equal(host(mod.__dict__, x, True), want)
+
+
+def test_a_changed_module_is_described_anew():
+    case = Case(256, 128, 128, 4, torch.bfloat16, seed=9, bias=True)
+    mod = case.module()
+    x = case.x(3).cuda()
+    first = mod(x)
+    assert torch.equal(mod(x), first)
+    mod.lut = (2 * mod.lut.float()).bfloat16()
+    assert pkg._lib.host.linear(mod.__dict__, x, True) is None
+    assert torch.equal(mod(x), mod._forward_route(x)) and not torch.equal(mod(x), first)
+    mod.bias.data = torch.zeros_like(mod.bias.data)
+    assert torch.equal(mod(x), mod._forward_route(x))
+    other = copy.deepcopy(mod)
+    assert torch.equal(other(x), mod(x))
+    mod.reference = True
+    assert rel_err(mod(x), mod._forward_route(x)) == 0.0 and pkg._lib.host.linear(mod.__dict__, x, True) is None
+    with torch.cuda.stream(torch.cuda.Stream()):
+        torch.cuda.current_stream().wait_stream(torch.cuda.default_stream())
+        assert torch.equal(other(x), other._forward_route(x))
+        torch.cuda.current_stream().synchronize()
+    with pytest.raises(ValueError, match="feature dim"):
+        other(x[:, :64])
+
+
+def test_scratch_of_a_captured_graph_is_its_own():
+    case = Case(1024, 512, 128, 4, torch.bfloat16, seed=12)
+    mod = case.module()
+    x = case.x(64).cuda()
+    want = mod(x)
+    graphs, outs = [], []
+    for _ in range(2):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            outs.append(mod(x))
+        graphs.append(g)
+    for g, o in zip(graphs * 2, outs * 2):
+        g.replay()
+        assert torch.equal(mod(x), want)
+        torch.cuda.synchronize()
+        assert torch.equal(o, want)
