@@ -66,6 +66,19 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
+// Phase test that may suspend the thread for a while (about a microsecond here) before it answers.
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(1000u)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait. `abort_flag` is a shared-memory word: once any waiter in the block has
 // timed out it is set, and every later wait returns at once, so a block that lost a
 // signal drains in microseconds. The deadline is in SM clock cycles. Returns false on
@@ -76,8 +89,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   if (*abort_flag) return false;
   const long long t0 = clock64();
   for (uint32_t i = 1;; ++i) {
-    if (mbar_test(bar, parity)) return true;
-    if ((i & 15u) == 0u) {
+    if (mbar_try(bar, parity)) return true;
+    if ((i & 3u) == 0u) {
       if (*abort_flag) return false;
       if (clock64() - t0 > limit) break;
     }
