@@ -47,11 +47,13 @@ enum {
                                     (4-bit codes, one stream, M <= 8, split = 0, no exchange). It
                                     is the library's choice for those shapes anyway, unless the
                                     process runs with B200LUT_GEMV_KERNEL=tile */
-  B200LUT_FLAG_CTA_PAIRS = 8     /* prefill GEMM: run launches of M >= 256 rows with an even number of
+  B200LUT_FLAG_CTA_PAIRS = 8,    /* prefill GEMM: run launches of M >= 256 rows with an even number of
                                     128-row tiles as pairs of CTAs (tcgen05 cta_group::2: one MMA
                                     covers 256 weight rows, each CTA fetches half of the activation
                                     tile; no multicast load). Same results bit for bit, measured
                                     slower than one CTA per tile, so it is never the default */
+  B200LUT_FLAG_WHOLE_TILES = 16  /* prefill GEMM: every output is one sum over all of K (no cut of K over
+                                    the blocks of a cluster) */
 };
 
 /* Epilogue selector of b200lut_gemv_multi / b200lut_gemm. */
@@ -405,6 +407,10 @@ int b200lut_gemm(const void* x, int64_t ldx, int M, int K, int dtype,
  * that return to zero by themselves), 16-byte aligned, and serves one launch at a time; it may
  * be reused across shapes. No counterpart in the reference (its GEMM is one tile per block). */
 size_t b200lut_gemm_workspace_bytes(int M, int N, int K);
+/* Scratch that a launch over N output rows in all makes use of: 0 where the kernel for batches and
+ * short prompts runs (it cuts K over thread-block clusters and exchanges sums in shared memory), else
+ * b200lut_gemm_workspace_bytes. */
+size_t b200lut_gemm_launch_workspace_bytes(int M, int N, int K, int bits, int group_size);
 int b200lut_gemm_ws(const void* x, int64_t ldx, int M, int K, int dtype,
                     const b200lut_segment* seg, int epilogue, int flags,
                     void* workspace, size_t workspace_bytes, void* stream);

@@ -24,6 +24,7 @@ FHT_FORWARD, FHT_ADJOINT, FHT_AWQ = 0, 1, 2
 FLAG_PDL = 1
 FLAG_TILE_KERNEL = 2     # decode GEMV: force the tile x K-split kernel
 FLAG_ROWS_KERNEL = 4     # decode GEMV: the row-range kernel where it serves the shapes
+FLAG_WHOLE_TILES = 16    # prefill GEMM: no cut of K
 FLAG_CTA_PAIRS = 8       # prefill GEMM: CTA pairs (tcgen05 cta_group::2); slower, never the default
 
 EXPORTS = (
@@ -31,7 +32,7 @@ EXPORTS = (
     "b200lut_repack_from_idxn", "b200lut_repack_to_idxn", "b200lut_unpack_codes",
     "b200lut_dequant", "b200lut_gemv_workspace_bytes", "b200lut_gemv_pick_split",
     "b200lut_gemv_multi", "b200lut_gemv", "b200lut_gemm", "b200lut_fht",
-    "b200lut_residual_project", "b200lut_residual_project_rows", "b200lut_silu_mul", "b200lut_gemm_workspace_bytes", "b200lut_gemm_ws", "b200lut_gemm_multi",
+    "b200lut_residual_project", "b200lut_residual_project_rows", "b200lut_silu_mul", "b200lut_gemm_workspace_bytes", "b200lut_gemm_launch_workspace_bytes", "b200lut_gemm_ws", "b200lut_gemm_multi",
     "b200lut_gemm_two_stream", "b200lut_gemm_two_stream_bytes",
     "b200lut_embed_gather", "b200lut_embed_gather_checked", "b200lut_round_rows", "b200lut_gemv_kgrouped",
     "b200lut_gemv_kgrouped_split", "b200lut_gemv_kgrouped_workspace_bytes", "b200lut_gemm_kgrouped", "b200lut_gemv_exchange", "b200lut_peer_export", "b200lut_peer_open", "b200lut_peer_close",
@@ -126,6 +127,8 @@ def lib() -> ctypes.CDLL:
                                      i32, vp, sz, i32, vp]
     L.b200lut_gemm_workspace_bytes.restype = sz
     L.b200lut_gemm_workspace_bytes.argtypes = [i32, i32, i32]
+    L.b200lut_gemm_launch_workspace_bytes.restype = sz
+    L.b200lut_gemm_launch_workspace_bytes.argtypes = [i32, i32, i32, i32, i32]
     L.b200lut_gemm_ws.restype = i32
     L.b200lut_gemm_ws.argtypes = [vp, i64, i32, i32, i32, ctypes.POINTER(Segment), i32, i32, vp, sz, vp]
     L.b200lut_gemm_multi.restype = i32
@@ -551,7 +554,11 @@ def gemm(x: torch.Tensor, seg, epilogue: int = EPI_NONE, flags: int = 0, split: 
     M, K = x.shape
     with _on_device(x.device):
         s0 = seg[0]
-        need = lib().b200lut_gemm_workspace_bytes(M, int(s0.N), K) if (split and not s0.packed2) else 0
+        need = 0
+        if not split:
+            flags |= FLAG_WHOLE_TILES
+        elif not s0.packed2:
+            need = lib().b200lut_gemm_launch_workspace_bytes(M, int(s0.N), K, int(s0.bits), int(s0.group_size))
         if need:
             ws = _gemm_workspace(x.device, need)
             check(lib().b200lut_gemm_ws(x.data_ptr(), x.stride(0), M, K, dtype_id(x.dtype), seg,
@@ -654,7 +661,11 @@ def gemm_multi(x: torch.Tensor, segs, nseg: int, flags: int = 0, split: bool = T
     M, K = x.shape
     with _on_device(x.device):
         total = sum(int(segs[i].N) for i in range(nseg))
-        need = lib().b200lut_gemm_workspace_bytes(M, total, K) if split else 0
+        need = 0
+        if split:
+            need = lib().b200lut_gemm_launch_workspace_bytes(M, total, K, int(segs[0].bits), int(segs[0].group_size))
+        else:
+            flags |= FLAG_WHOLE_TILES
         ws = _gemm_workspace(x.device, need) if need else None
         check(lib().b200lut_gemm_multi(x.data_ptr(), x.stride(0), M, K, dtype_id(x.dtype), segs, nseg,
                                        flags, ptr(ws), ws.numel() if ws is not None else 0, _stream(x)))

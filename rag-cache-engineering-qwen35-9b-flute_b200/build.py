@@ -16,7 +16,7 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libb200lut.so")
 HOST = os.path.join(HERE, "_b200lut_host.so")      # native host layer (torch C++), links LIB
-SOURCES = ("api.cu", "layout.cu", "gemv.cu", "fht.cu", "gemm_tc.cu", "peer.cu", "residual.cu", "elementwise.cu", "embed.cu", "gemv_kgrouped.cu")
+SOURCES = ("api.cu", "layout.cu", "gemv.cu", "fht.cu", "gemm_tc.cu", "gemm_cluster.cu", "peer.cu", "residual.cu", "elementwise.cu", "embed.cu", "gemv_kgrouped.cu")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
 

@@ -91,6 +91,12 @@ template <> struct DType<__half> {
 
 // Status word of the decode kernels' exchange waits (defined with the GEMV): value and clear.
 int exchange_status_take();
+// Status word of the batched-decode tensor-core GEMM: value and clear.
+int gemm_cluster_status_take();
+// That GEMM (gemm_cluster.cu); *served is false, and nothing has been launched, for shapes it does not take.
+int cluster_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b200lut_segment* segs, int nseg, bool pdl,
+                 void* stream, float* acc_out, const float* acc_in, long long ld_acc, long long wait_cycles, bool whole_tiles, bool* served);
+bool cluster_gemm_serves(int M, int row_tiles, int K, int bits, int group_size);
 // Status word of the embedding gather (an id outside the table): value and clear.
 int embed_status_take();
 

@@ -23,9 +23,7 @@
 
 #include <cstdlib>
 
-#include "common.cuh"
-#include "pairtable.cuh"
-#include "tc05.cuh"
+#include "gemm_parts.cuh"
 
 namespace b200lut {
 namespace {
@@ -57,15 +55,6 @@ struct GemmParams {
   uint32_t smem_bytes;
   int out_aligned;   // out rows are 16-byte aligned: staged, vectorised epilogue
 };
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar,
-                                            int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      :
-      : "r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
-      : "memory");
-}
 
 // The same for a CTA of a pair (cta_group::2): the tile lands in this CTA's shared memory, its
 // bytes are reported to `bar`, which may be the other CTA's barrier. Not a multicast load.
@@ -332,21 +321,6 @@ constexpr int kPStages = 4;             // ring depth of both operands
 constexpr uint32_t kPACol = 256;        // operand stage s at columns [256 + 32 s, 288 + 32 s)
 constexpr int kPStageTokens = 48;       // tokens per staged epilogue slice (12 KB per column half)
 
-constexpr int kPMaxSeg = 4;             // projections that share x in one launch (Q/K/V/z, gate/up)
-
-// One projection of a launch: its row tiles are the global row tiles [row0, next row0).
-struct PersistSeg {
-  const uint8_t* packed;
-  const uint16_t* lut;
-  const uint16_t* bias;
-  uint16_t* out;
-  long long ldo;
-  int row0, n_groups, out_aligned;
-  int res_rank;            // rank of the low-rank residual, 0 if the projection has none
-  const uint16_t* resA;    // [N, res_rank], row-major
-  int t_col0, pad;         // first column of this projection's block of the t matrix
-};
-
 struct PersistParams {
   PersistSeg seg[kPMaxSeg];
   int nsegs;
@@ -406,34 +380,6 @@ __device__ __forceinline__ void load_slab_pair(uint32_t (&w)[2 * BITS], const ui
   }
 }
 
-// Pair-table address of field i (0..15) of local slab sl (0, 1): the field's 2 * BITS bits
-// moved to address bits 8.., joined with the lane base.
-template <int BITS>
-__device__ __forceinline__ uint32_t slab_field_addr(const uint32_t (&w)[2 * BITS], int sl, int i,
-                                                    uint32_t base) {
-  if constexpr (BITS == 4) {
-    return __byte_perm(w[4 * sl + (i >> 2)], base, 0x7604u | (uint32_t(i & 3) << 4));
-  } else {
-    constexpr uint32_t kMask = ((1u << (2 * BITS)) - 1u) << 8;
-    const int pos = 32 * BITS * sl + 2 * BITS * i, m = pos >> 5, sh = pos & 31;
-    uint32_t v;
-    if (sh + 2 * BITS > 32) v = __funnelshift_r(w[m], w[(m + 1) % (2 * BITS)], sh - 8);
-    else if (sh >= 8) v = w[m] >> (sh - 8);
-    else v = w[m] << (8 - sh);
-    return (v & kMask) | base;
-  }
-}
-
-// The projection that owns global row tile `row` (static indexing of the parameter block: a
-// chain of selects, no local copy).
-__device__ __forceinline__ PersistSeg segment_of_row(const PersistParams& p, int row) {
-  PersistSeg sd = p.seg[0];
-#pragma unroll
-  for (int i = 1; i < kPMaxSeg; ++i)
-    if (i < p.nsegs && row >= p.seg[i].row0) sd = p.seg[i];
-  return sd;
-}
-
 // First tile of block b when the tile list is cut into gridDim.x ranges of equal cost
 // (cost of a tile = its token columns).
 __device__ __forceinline__ int persist_first_tile(const PersistParams& p, long long b, long long nb) {
@@ -456,15 +402,6 @@ __device__ __forceinline__ int persist_first_tile(const PersistParams& p, long l
 //                  with the codes) and reads every weight with one 16-bit load; the rest of the
 //                  pipeline does not know the difference.
 constexpr int kModePlain = 0, kModeResidual = 1, kModeKGrouped = 2;
-
-// The 2 * BITS bits of field i (0..15) of local slab sl (0, 1): two codes, the lower one first.
-template <int BITS>
-__device__ __forceinline__ uint32_t slab_field(const uint32_t (&w)[2 * BITS], int sl, int i) {
-  constexpr uint32_t kMask = (1u << (2 * BITS)) - 1u;
-  const int pos = 32 * BITS * sl + 2 * BITS * i, m = pos >> 5, sh = pos & 31;
-  if (sh + 2 * BITS > 32) return __funnelshift_r(w[m], w[(m + 1) % (2 * BITS)], sh) & kMask;
-  return (w[m] >> sh) & kMask;
-}
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -1002,23 +939,6 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap xmap,
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      p = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
-
 template <typename T>
 int launch(const CUtensorMap& map, const GemmParams& p, int n_tiles, bool pdl, cudaStream_t stream) {
   auto kern = gemm_tc_kernel<T>;
@@ -1108,22 +1028,6 @@ int launch_persistent(const CUtensorMap& map, const CUtensorMap& tmap, const Per
 // tiles are worth it, the row tiles must pair up, and so must the SMs.
 bool pairs_serve(int rows, int M, int sms) { return M >= kPMaxNT && rows >= 2 && rows % 2 == 0 && sms % 2 == 0; }
 
-int encode_x_map(CUtensorMap* map, const void* x, int64_t ldx, int M, int K, int dtype, int NT) {
-  EncodeTiledFn enc = encode_fn();
-  B200LUT_REQUIRE(enc != nullptr, B200LUT_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-  const cuuint64_t dims[2] = {cuuint64_t(K), cuuint64_t(M)};
-  const cuuint64_t strides[1] = {cuuint64_t(ldx) * 2};
-  const cuuint32_t box[2] = {cuuint32_t(kChunkK), cuuint32_t(NT)};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = enc(map, dtype == B200LUT_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
-                                                     : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                         2, const_cast<void*>(x), dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  B200LUT_REQUIRE(r == CUDA_SUCCESS, B200LUT_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", int(r));
-  return B200LUT_OK;
-}
-
 }  // namespace
 
 }  // namespace b200lut
@@ -1140,18 +1044,51 @@ extern "C" int b200lut_device_status(void) {
   if (v != 0) cudaMemcpyToSymbol(g_gemm_status, &zero, sizeof(int));
   const int e = b200lut::exchange_status_take();
   const int g = b200lut::embed_status_take();
-  return v != 0 ? v : (e != 0 ? e : g);
+  const int c = b200lut::gemm_cluster_status_take();
+  return v != 0 ? v : (c != 0 ? c : (e != 0 ? e : g));
 }
 
 namespace {
+constexpr int kClusterMaxM = 1024;
+constexpr long long kClusterMaxTiles = 640;
+
+bool cluster_serves(int M, long long row_tiles, int K, int bits, int group_size) {
+  return M < kClusterMaxM && row_tiles * ((M + 127) / 128) <= kClusterMaxTiles && group_size >= 64 &&
+         cluster_gemm_serves(M, int(row_tiles), K, bits, group_size);
+}
+
 // Host side of the persistent kernel: `nseg` projections that share x (one code stream each,
 // the same code width and group size, at most two palettes per 128-row tile) as one launch
 // whose row tiles are the concatenation of the projections' row tiles.
 int persistent_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b200lut_segment* segs,
-                    int nseg, bool pdl, void* workspace, size_t workspace_bytes,
+                    int nseg, int flags, void* workspace, size_t workspace_bytes,
                     void* stream, float* acc_out = nullptr, const float* acc_in = nullptr,
-                    long long ld_acc = 0, int kg_rows = 0, bool cta_pairs = false) {
+                    long long ld_acc = 0, int kg_rows = 0) {
+  // Waits inside the kernel give up after ~10 ms. A profiler that replays the kernel with
+  // heavy instrumentation can stretch a healthy wait beyond that; B200LUT_WAIT_MS raises the
+  // bound for such runs (capped at one second).
   PersistParams pp = {};
+  pp.wait_cycles = tc::kWaitCycles;
+  if (const char* e = getenv("B200LUT_WAIT_MS")) {
+    long ms = atol(e);
+    if (ms < 1) ms = 1;
+    if (ms > 1000) ms = 1000;
+    pp.wait_cycles = (long long)ms * 2000000ll;
+  }
+  const bool pdl = (flags & B200LUT_FLAG_PDL) != 0, cta_pairs = (flags & B200LUT_FLAG_CTA_PAIRS) != 0;
+  {
+    // Up to about four 128-token tiles per SM the cluster kernel is ahead (24576 x 4096: 24.7 against
+    // 37.1 us at 64 tokens, 65.7 against 86.9 at 384, even at 512; 4096 x 4096: 8.7 / 15.4 at 64, 15.1
+    // / 27.3 at 256, 27.1 / 33.4 at 768); beyond, both are held by the power cap.
+    long long row_tiles = 0;
+    for (int i = 0; i < nseg; ++i) row_tiles += segs[i].N / kTileRows;
+    if (kg_rows == 0 && !(flags & B200LUT_FLAG_CTA_PAIRS) && cluster_serves(M, row_tiles, K, segs[0].bits, segs[0].group_size)) {
+      bool served = false;
+      const int rc = cluster_gemm(x, ldx, M, K, dtype, segs, nseg, pdl, stream, acc_out, acc_in, ld_acc, pp.wait_cycles,
+                                  (flags & B200LUT_FLAG_WHOLE_TILES) != 0, &served);
+      if (rc != B200LUT_OK || served) return rc;
+    }
+  }
   pp.acc_out = acc_out; pp.acc_in = acc_in; pp.ld_acc = ld_acc;
   const bool kgrouped = kg_rows > 0;     // segs[0].lut is lut_k [K / 128][kg_rows][2^bits]
   pp.kg_N = kg_rows;
@@ -1206,16 +1143,6 @@ int persistent_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b
   pp.n_tiles = pair ? rows / 2 : rows;      // a pair schedules pairs of row tiles
   pp.W = (pp.m_tiles - 1) * pp.NT + ((M - (pp.m_tiles - 1) * pp.NT + 31) / 32) * 32;
   pp.smem_bytes = uint32_t(kMaxDynSmem);
-  // Waits inside the kernel give up after ~10 ms. A profiler that replays the kernel with
-  // heavy instrumentation can stretch a healthy wait beyond that; B200LUT_WAIT_MS raises the
-  // bound for such runs (capped at one second).
-  pp.wait_cycles = tc::kWaitCycles;
-  if (const char* e = getenv("B200LUT_WAIT_MS")) {
-    long ms = atol(e);
-    if (ms < 1) ms = 1;
-    if (ms > 1000) ms = 1000;
-    pp.wait_cycles = (long long)ms * 2000000ll;
-  }
   CUtensorMap pmap, tmap;
   const int box_rows = pair ? pp.NT / 2 : pp.NT;     // each CTA of a pair fetches half of the tile's tokens
   if (int rc = encode_x_map(&pmap, x, ldx, M, K, dtype, box_rows)) return rc;
@@ -1297,6 +1224,11 @@ extern "C" size_t b200lut_gemm_workspace_bytes(int M, int N, int K) {
   return need;
 }
 
+extern "C" size_t b200lut_gemm_launch_workspace_bytes(int M, int N, int K, int bits, int group_size) {
+  if (M >= 1 && N >= kTileRows && cluster_serves(M, N / kTileRows, K, bits, group_size)) return 0;
+  return b200lut_gemm_workspace_bytes(M, N, K);
+}
+
 extern "C" int b200lut_gemm(const void* x, int64_t ldx, int M, int K, int dtype,
                             const b200lut_segment* seg, int epilogue, int flags, void* stream) {
   return b200lut_gemm_ws(x, ldx, M, K, dtype, seg, epilogue, flags, nullptr, 0, stream);
@@ -1327,9 +1259,7 @@ extern "C" int b200lut_gemm_multi(const void* x, int64_t ldx, int M, int K, int 
                     "one group size >= 64 (segment %d: %d bits, group %d)", i, s.bits, s.group_size);
     B200LUT_REQUIRE(aligned16(s.packed), B200LUT_ERR_ALIGN, "code buffers must be 16-byte aligned");
   }
-  return persistent_gemm(x, ldx, M, K, dtype, segs, nseg, (flags & 1) != 0, workspace,
-                         workspace_bytes, stream, nullptr, nullptr, 0, 0,
-                         (flags & B200LUT_FLAG_CTA_PAIRS) != 0);
+  return persistent_gemm(x, ldx, M, K, dtype, segs, nseg, flags, workspace, workspace_bytes, stream);
 }
 
 extern "C" int b200lut_gemm_kgrouped(const void* x, int64_t ldx, int M, int K, int dtype,
@@ -1358,8 +1288,8 @@ extern "C" int b200lut_gemm_kgrouped(const void* x, int64_t ldx, int M, int K, i
   s.group_size = kTileRows;     // not used by the K-grouped lookup
   s.n_groups = N / kTileRows;
   s.bits = bits;
-  return persistent_gemm(x, ldx, M, K, dtype, &s, 1, (flags & 1) != 0, workspace, workspace_bytes, stream,
-                         nullptr, nullptr, 0, N, (flags & B200LUT_FLAG_CTA_PAIRS) != 0);
+  return persistent_gemm(x, ldx, M, K, dtype, &s, 1, flags, workspace, workspace_bytes, stream,
+                         nullptr, nullptr, 0, N);
 }
 
 extern "C" size_t b200lut_gemm_two_stream_bytes(int M, int N) {
@@ -1396,11 +1326,10 @@ extern "C" int b200lut_gemm_two_stream(const void* x, int64_t ldx, int M, int K,
   first.res_rank = 0; first.resA = nullptr; first.res_t = nullptr;   // the second launch carries it
   second.packed = s.packed2; second.lut = s.lut2; second.bits = s.bits2;
   second.packed2 = second.lut2 = nullptr; second.bits2 = 0;
-  const bool pdl = (flags & 1) != 0;
-  if (int rc = persistent_gemm(x, ldx, M, K, dtype, &first, 1, pdl, nullptr, 0, stream, acc,
+  if (int rc = persistent_gemm(x, ldx, M, K, dtype, &first, 1, flags & B200LUT_FLAG_PDL, nullptr, 0, stream, acc,
                                nullptr, s.N))
     return rc;
-  return persistent_gemm(x, ldx, M, K, dtype, &second, 1, pdl, nullptr, 0, stream, nullptr, acc,
+  return persistent_gemm(x, ldx, M, K, dtype, &second, 1, flags & B200LUT_FLAG_PDL, nullptr, 0, stream, nullptr, acc,
                          s.N);
 }
 
@@ -1431,8 +1360,7 @@ extern "C" int b200lut_gemm_ws(const void* x, int64_t ldx, int M, int K, int dty
   const bool pdl = (flags & 1) != 0;
   const int nl = s.group_size >= 128 ? 1 : 128 / s.group_size;
   if (!two && nl <= 2 && K / kChunkK >= 2) {
-    return persistent_gemm(x, ldx, M, K, dtype, seg, 1, pdl, workspace, workspace_bytes, stream,
-                           nullptr, nullptr, 0, 0, (flags & B200LUT_FLAG_CTA_PAIRS) != 0);
+    return persistent_gemm(x, ldx, M, K, dtype, seg, 1, flags, workspace, workspace_bytes, stream);
   }
 
   // what is left for the one-tile kernel: two code streams, the fused gate/up form, four

@@ -129,7 +129,7 @@ inline int64_t padded_cols(int rank) { return 64 * ((int64_t(rank) + 63) / 64); 
 
 // `n` projections that share x as one prefill launch, with the split schedule's scratch.
 inline void gemm_launch(const Rows& r, int K, int dtype, const b200lut_segment* segs, int n, int64_t rows, const Ctx& c) {
-  const size_t need = segs[0].packed2 ? 0 : b200lut_gemm_workspace_bytes(r.M, int(rows), K);
+  const size_t need = segs[0].packed2 ? 0 : b200lut_gemm_launch_workspace_bytes(r.M, int(rows), K, segs[0].bits, segs[0].group_size);
   at::Tensor ws;
   if (need) ws = scratch_pool().get(Scratch::kSplit, c.device, c.stream, need);
   void* wp = need ? ws.mutable_data_ptr() : nullptr;

@@ -83,9 +83,11 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 // timed out it is set, and every later wait returns at once, so a block that lost a
 // signal drains in microseconds. The deadline is in SM clock cycles. Returns false on
 // abort.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          int* status, int why, long long limit = kWaitCycles) {
-  if (mbar_test(bar, parity)) return true;
+// The waiting part is a function of its own: a role's loop then fits the instruction cache of its
+// scheduler (with the wait inlined a dozen times the roles of one block evicted each other's loops,
+// 7 to 10 cycles per instruction in a single-thread role).
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                            int* status, int why, long long limit) {
   if (*abort_flag) return false;
   const long long t0 = clock64();
   for (uint32_t i = 1;; ++i) {
@@ -94,6 +96,34 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
       if (*abort_flag) return false;
       if (clock64() - t0 > limit) break;
     }
+  }
+  *abort_flag = 1;
+  if (status) atomicCAS(status, kStatusOk, why);
+  return false;
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                          int* status, int why, long long limit = kWaitCycles) {
+  if (mbar_test(bar, parity)) return true;
+  return mbar_wait_slow(bar, parity, abort_flag, status, why, limit);
+}
+
+// The same for arrivals of other CTAs of the cluster: what they wrote into this CTA's shared memory
+// before they arrived is visible after the wait.
+static __device__ __noinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                                  int* status, int why, long long limit) {
+  const long long t0 = clock64();
+  for (uint32_t i = 0;; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(1000u)
+        : "memory");
+    if (ok) return true;
+    if (*abort_flag) return false;
+    if (clock64() - t0 > limit) break;
   }
   *abort_flag = 1;
   if (status) atomicCAS(status, kStatusOk, why);
@@ -228,6 +258,17 @@ constexpr uint32_t kPeerBitMask = 0xFEFFFFFFu;
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_id() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
   return r;
 }
 __device__ __forceinline__ void cluster_sync() {

@@ -1,0 +1,71 @@
+"""The tensor-core GEMM for batches and short prompts (csrc/gemm_cluster.cu) where it can go wrong: token
+counts at the edges of its 16- to 128-token tiles, odd and few k-blocks per CTA, every cut of K its
+planner picks (few row tiles: up to eight CTAs per cluster), two palettes per tile, every code width,
+merged projections, residual k-blocks that start in the middle of a stage, unaligned outputs."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from helpers import TOL, Case, pkg, rel_err
+
+pytestmark = pytest.mark.gpu
+L = pkg._lib
+
+
+@pytest.fixture(autouse=True)
+def _no_device_error():
+    yield
+    torch.cuda.synchronize()
+    assert L.lib().b200lut_device_status() == 0
+
+
+@pytest.mark.parametrize("N,K,gs,bits,dtype,M,opts", (
+    (128, 128, 128, 4, torch.bfloat16, 17, {}),                       # two k-blocks, one tile
+    (128, 4160, 128, 4, torch.bfloat16, 33, {}),                      # 65 k-blocks over eight CTAs
+    (256, 2112, 64, 4, torch.float16, 128, dict(bias=True)),          # 33 k-blocks, two palettes, a full tile
+    (384, 1984, 128, 3, torch.bfloat16, 129, {}),                     # 31 k-blocks, two token tiles
+    (640, 1024, 64, 3, torch.float16, 250, dict(bias=True)),
+    (256, 1536, 256, 2, torch.bfloat16, 64, {}),
+    (512, 320, 512, 1, torch.float16, 65, dict(bias=True)),           # five k-blocks
+    (128, 2048, 128, 4, torch.bfloat16, 48, dict(residual=32)),
+    (256, 1088, 64, 4, torch.float16, 100, dict(residual=72, bias=True)),   # 17 k-blocks, two residual blocks
+    (384, 192, 128, 4, torch.bfloat16, 20, dict(residual=8)),         # the residual opens a stage after three k-blocks
+    (19200, 128, 128, 4, torch.bfloat16, 31, {}),                     # 150 row tiles: more than one per CTA
+    (1280, 128, 128, 4, torch.float16, 900, {}),                      # 80 tiles of eight token tiles
+))
+def test_forward_matches_oracle(N, K, gs, bits, dtype, M, opts):
+    case = Case(N, K, gs, bits, dtype, seed=N + 3 * K + M, **opts)
+    mod = case.module()
+    x = case.x(M).cuda()
+    got = mod(x)
+    assert rel_err(got, case.oracle(case.x(M))) <= TOL
+    assert torch.equal(mod(x), got)                                    # ascending-k exchange: deterministic
+
+
+@pytest.mark.parametrize("M", (24, 127))
+def test_cut_and_whole_tiles_agree(M):
+    # the same products in fp32, summed in parts: n terms in any order differ by at most n * 2^-24 of the
+    # sum of magnitudes; here that is far below one bf16 rounding (2^-8 of the largest value, rel_err's scale)
+    case = Case(256, 4096, 128, 4, torch.bfloat16, seed=M)
+    mod = case.module()
+    mod._ensure_packed()
+    x = case.x(M).cuda()
+    outs = []
+    for split in (True, False):
+        o = torch.full((M, 256 + 3), float("nan"), dtype=case.dtype, device="cuda")     # odd stride: unaligned rows
+        L.gemm(x, L.make_segments([dict(packed=mod._packed, lut=mod.lut, N=256, group_size=128, n_groups=2, bits=4,
+                                        out=o, ldo=259)]), split=split)
+        assert torch.isnan(o[:, 256:].float()).all()
+        outs.append(o[:, :256])
+    assert rel_err(outs[0], outs[1].cpu()) <= 2.0 ** -8
+    assert rel_err(outs[0], case.oracle(case.x(M))) <= TOL
+
+
+def test_merged_projections_with_and_without_a_residual():
+    K, M, dt = 1344, 40, torch.float16                                 # 21 k-blocks
+    cases = [Case(n, K, 128, 4, dt, seed=80 + i, bias=(i == 0), residual=16 * i) for i, n in enumerate((256, 128, 384))]
+    qkv = pkg.SplitQKV(*(c.module() for c in cases))
+    x = cases[0].x(M)
+    want = torch.cat([c.oracle(x) for c in cases], dim=-1)
+    assert rel_err(qkv(x.cuda()), want) <= TOL
