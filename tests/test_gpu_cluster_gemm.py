@@ -46,7 +46,8 @@ def test_forward_matches_oracle(N, K, gs, bits, dtype, M, opts):
 @pytest.mark.parametrize("M", (24, 127))
 def test_cut_and_whole_tiles_agree(M):
     # the same products in fp32, summed in parts: n terms in any order differ by at most n * 2^-24 of the
-    # sum of magnitudes; here that is far below one bf16 rounding (2^-8 of the largest value, rel_err's scale)
+    # sum of magnitudes, far below one bf16 step; so the two roundings give the same or neighbouring values,
+    # and neighbours in bf16 (8 significant bits) lie at most 2^-7 of their size apart
     case = Case(256, 4096, 128, 4, torch.bfloat16, seed=M)
     mod = case.module()
     mod._ensure_packed()
@@ -58,7 +59,7 @@ def test_cut_and_whole_tiles_agree(M):
                                         out=o, ldo=259)]), split=split)
         assert torch.isnan(o[:, 256:].float()).all()
         outs.append(o[:, :256])
-    assert rel_err(outs[0], outs[1].cpu()) <= 2.0 ** -8
+    assert rel_err(outs[0], outs[1].cpu()) <= 2.0 ** -7
     assert rel_err(outs[0], case.oracle(case.x(M))) <= TOL
 
 
