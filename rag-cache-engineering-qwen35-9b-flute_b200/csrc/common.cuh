@@ -95,7 +95,10 @@ int exchange_status_take();
 int gemm_cluster_status_take();
 // That GEMM (gemm_cluster.cu); *served is false, and nothing has been launched, for shapes it does not take.
 int cluster_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b200lut_segment* segs, int nseg, bool pdl,
-                 void* stream, float* acc_out, const float* acc_in, long long ld_acc, long long wait_cycles, bool whole_tiles, bool* served);
+                 void* stream, float* acc_out, const float* acc_in, long long ld_acc, long long wait_cycles, bool whole_tiles, bool gated,
+                 bool* served);
+// The bound of the tensor-core kernels' in-kernel waits, in SM clock cycles (B200LUT_WAIT_MS raises it).
+long long gemm_wait_cycles();
 bool cluster_gemm_serves(int M, int row_tiles, int K, int bits, int group_size);
 // Status word of the embedding gather (an id outside the table): value and clear.
 int embed_status_take();

@@ -1,4 +1,4 @@
-// LUT GEMM for batches of about 9 to a few hundred rows (batched decode, short prompts) on tcgen05.
+// LUT GEMM for batches of 9 to a few hundred rows (batched decode, short prompts) on tcgen05.
 //
 // Such a launch is a stream of codes with little arithmetic per code: at 64 rows a 128 x 64 chunk of
 // 4-bit codes (4 KB of HBM, 177 cycles of an SM's share) feeds four MMAs of 128 x 64 x 16 (149
@@ -21,8 +21,13 @@
 // Weights are the A operand in tensor memory, tokens (up to 128 per tile) the B operand in shared
 // memory, as in gemm_tc.cu. All waits are bounded.
 //
+// The gated form (kModeGated, up to 16 tokens): a cluster takes a row tile of gate and then the same row
+// tile of up, and an epilogue thread, which finishes the same eight outputs of both, holds the finished
+// gate values in registers: silu(gate) * up stays fp32 until its one rounding, as in the decode kernels.
+//
 // Warps: 0-15 lookup (row quarter = warp % 4; every fourth stage of two chunks belongs to group warp / 4),
 // 16 code producer, 17 activation producer, 18 MMA issuer, 19-26 epilogue.
+#include <cstdlib>
 #include <mutex>
 
 #include "gemm_parts.cuh"
@@ -60,7 +65,8 @@ constexpr uint32_t kCWindowEnd = 1024 + kCDynBytes;
 
 struct ClusterParams {
   // what every role reads first, close together: a launch's parameters start out in no cache
-  int split, clusters, tiles_each, tiles_more;   // CTAs per cluster; clusters; whole share of tiles, clusters with one more
+  int split, clusters, tiles_each, tiles_more;   // CTAs per cluster; clusters; whole share of tiles (gated form:
+                                                 // pairs of tiles), clusters with one more
   int kb_each, kb_more;                          // k-blocks per CTA of a cluster, CTAs (the first ones) with one more
   int quads_each, quads_more;                    // token quads that a CTA finishes, likewise
   int NT, m_tiles, G, gs, M, nx, nc;             // tokens per tile, token tiles, ..., activation slots, code slots
@@ -156,10 +162,14 @@ __device__ __forceinline__ void load_codes(uint32_t (&w)[2 * BITS], uint32_t slo
 }
 
 
-template <typename T, int BITS, bool RES>
+constexpr int kModePlain = 0, kModeResidual = 1, kModeGated = 2;
+constexpr int kCGatedMaxNT = 16;          // one piece of eight outputs per epilogue thread and tile
+
+template <typename T, int BITS, int MODE>
 __global__ void __launch_bounds__(kCThreads, 1)
 gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap tmap,
                                    const ClusterParams p) {
+  constexpr bool RES = MODE == kModeResidual, GATED = MODE == kModeGated;
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t low = smem_u32(smem) & kCWindowMask, win = smem_u32(smem) - low;
@@ -180,15 +190,20 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
   const int lenc = !RES || c0 + len <= p.G ? len : (p.G > c0 ? p.G - c0 : 0);  // with codes,
   const int lenr = len - lenc;                                                 // and the residual's, which close the tile
   const int pc = (lenc + 1) & ~1, lp = pc + ((lenr + 1) & ~1);                 // both start a stage of their own
-  const int t0 = cid * p.tiles_each + (cid < p.tiles_more ? cid : p.tiles_more);
+  constexpr int kUnit = GATED ? 2 : 1;             // tiles of a unit of the schedule
+  const int t0 = kUnit * (cid * p.tiles_each + (cid < p.tiles_more ? cid : p.tiles_more));
   // Never seen: the layout starts at the window's first dynamic byte. Such a CTA does no work.
   const bool bad_window = low != 1024;
-  const int ntile = bad_window ? 0 : p.tiles_each + (cid < p.tiles_more ? 1 : 0);
+  const int ntile = bad_window ? 0 : kUnit * (p.tiles_each + (cid < p.tiles_more ? 1 : 0));
   const long long lim = p.wait_cycles;
   int nl = kTileRows / p.gs;
   if (nl < 1) nl = 1;
-  auto row_of = [&](int tile) { return p.m_tiles == 1 ? tile : tile / p.m_tiles; };
-  auto tok_of = [&](int tile) { return p.m_tiles == 1 ? 0 : (tile % p.m_tiles) * p.NT; };
+  // the gated form has one token tile, and tiles 2r and 2r + 1 are row tile r of gate and of up
+  auto row_of = [&](int tile) {
+    if constexpr (GATED) return (tile & 1 ? p.seg[1].row0 : 0) + (tile >> 1);
+    else return p.m_tiles == 1 ? tile : tile / p.m_tiles;
+  };
+  auto tok_of = [&](int tile) { return GATED || p.m_tiles == 1 ? 0 : (tile % p.m_tiles) * p.NT; };
 
   asm volatile("griddepcontrol.launch_dependents;");
   // The code producer sets up its own barriers and does not wait for the block: its first copies are
@@ -423,15 +438,16 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
     float* acc_out = p.acc_out;
     const float* acc_in = p.acc_in;
     pin(acc_out); pin(acc_in);
+    float gate[8];                                                 // gated form: what the last (gate) tile came to
     for (int t = 0; t < ntile; ++t) {
       const int row = row_of(t0 + t), m0 = tok_of(t0 + t);
       const PersistSeg sd = segment_of_row(p, row);
       const int n = (row - sd.row0) * kTileRows + 32 * q;          // first of the warp's 32 rows
-      uint16_t* out = sd.out + n;
-      long long ldo = sd.ldo;
+      uint16_t* out = (GATED ? p.seg[0].out : sd.out) + n;
+      long long ldo = GATED ? p.seg[0].ldo : sd.ldo;
       int M = p.M;
       pin(out); pin(ldo); pin(M);
-      const bool vec = sd.out_aligned != 0;
+      const bool vec = (GATED ? p.seg[0].out_aligned : sd.out_aligned) != 0;
       const float bias = sd.bias ? DType<T>::to_float(sd.bias[n + lane]) : 0.f;
       const uint32_t acc = tmem + (uint32_t(32 * q) << 16) + uint32_t(t & 1) * kCMaxNT;
       if (S > 1 && warp == kCEpiWarp && lane == 0)                 // what the others will write here for this tile
@@ -487,15 +503,26 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
             }
           }
         }
+        if constexpr (GATED) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] += bias;
+          if ((t & 1) == 0) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) gate[j] = v[j];
+            continue;
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = gate[j] / (1.f + __expf(-gate[j])) * v[j];
+        }
         const int tok0 = m0 + 4 * b, most = both ? 8 : 4;
         const int ntok = M - tok0 < most ? M - tok0 : most;         // tokens of this piece that exist
-        if (acc_out) {                             // first stream of two: raw fp32 sums
+        if (!GATED && acc_out) {                   // first stream of two: raw fp32 sums
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             if (j < ntok) __stcg(acc_out + (tok0 + j) * p.ld_acc + n + lane, v[j]);
           continue;
         }
-        if (acc_in) {
+        if (!GATED && acc_in) {
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             if (j < ntok) v[j] += __ldcg(acc_in + (tok0 + j) * p.ld_acc + n + lane);
@@ -506,7 +533,7 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             asm volatile("st.shared.u16 [%0], %1;" ::"r"(stage + uint32_t(j * 64 + lane * 2)),
-                         "h"(DType<T>::from_float(v[j] + bias))
+                         "h"(DType<T>::from_float(GATED ? v[j] : v[j] + bias))
                          : "memory");
           __syncwarp();
           const int j = lane >> 2;
@@ -514,7 +541,7 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
         } else {
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            if (j < ntok) out[(tok0 + j) * ldo + lane] = DType<T>::from_float(v[j] + bias);
+            if (j < ntok) out[(tok0 + j) * ldo + lane] = DType<T>::from_float(GATED ? v[j] : v[j] + bias);
         }
       }
       tc::fence_before_sync();
@@ -596,22 +623,22 @@ int encode_x_map3(CUtensorMap* map, const void* x, int64_t ldx, int M, int K, in
   return B200LUT_OK;
 }
 
-template <typename T, int BITS, bool RES>
+template <typename T, int BITS, int MODE>
 int configure(int dev) {
   static bool done[64] = {false};
   if (dev < 64 && done[dev]) return B200LUT_OK;
-  auto kern = gemm_tc_persistent_kernel_clusters<T, BITS, RES>;
+  auto kern = gemm_tc_persistent_kernel_clusters<T, BITS, MODE>;
   B200LUT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCDynBytes)));
   if (dev < 64) done[dev] = true;
   return B200LUT_OK;
 }
 
-template <typename T, int BITS, bool RES>
+template <typename T, int BITS, int MODE>
 int launch_cluster(const CUtensorMap& xmap, const CUtensorMap& tmap, const ClusterParams& p, uint32_t smem, bool pdl,
                    cudaStream_t stream) {
   int dev = 0;
   B200LUT_CUDA_OK(cudaGetDevice(&dev));
-  if (int rc = configure<T, BITS, RES>(dev)) return rc;
+  if (int rc = configure<T, BITS, MODE>(dev)) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(p.clusters * p.split), 1, 1);
   cfg.blockDim = dim3(kCThreads, 1, 1);
@@ -633,7 +660,7 @@ int launch_cluster(const CUtensorMap& xmap, const CUtensorMap& tmap, const Clust
   }
   cfg.attrs = attr;
   cfg.numAttrs = unsigned(na);
-  auto kern = gemm_tc_persistent_kernel_clusters<T, BITS, RES>;
+  auto kern = gemm_tc_persistent_kernel_clusters<T, BITS, MODE>;
   B200LUT_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, xmap, tmap, p));
   return B200LUT_OK;
 }
@@ -650,8 +677,8 @@ int max_clusters(int split) {
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return 0;
   if (split == 1) return n = sms;
-  auto kern = gemm_tc_persistent_kernel_clusters<__nv_bfloat16, 4, false>;
-  if (configure<__nv_bfloat16, 4, false>(dev) != B200LUT_OK) return 0;
+  auto kern = gemm_tc_persistent_kernel_clusters<__nv_bfloat16, 4, kModePlain>;
+  if (configure<__nv_bfloat16, 4, kModePlain>(dev) != B200LUT_OK) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(split), 1, 1);
   cfg.blockDim = dim3(kCThreads, 1, 1);
@@ -674,8 +701,9 @@ int max_clusters(int split) {
 // The cut of K that finishes first, by a fit (microseconds) to launches measured at 2048 to 24576 rows,
 // K = 4096 and 12288, 24 to 1024 tokens, cuts of 1 to 8: a k-block of the busiest cluster, what a launch
 // costs besides, what the exchange adds, and what is lost when the launch fills more than half of the
-// SMs (below that, its start and end run beside its neighbours' in the stream).
-bool plan_cluster(int M, int rows, int Gx, int bits, int group_size, bool whole_tiles, ClusterPlan* best) {
+// SMs (below that, its start and end run beside its neighbours' in the stream). `unit` tiles go to a
+// cluster together; c.tiles counts units.
+bool plan_cluster(int M, int rows, int Gx, int bits, int group_size, bool whole_tiles, int unit, ClusterPlan* best) {
   const int m_tiles = (M + kCMaxNT - 1) / kCMaxNT;
   const int per = (M + m_tiles - 1) / m_tiles, NT = (per + 15) / 16 * 16;
   const int sms = max_clusters(1);
@@ -685,11 +713,11 @@ bool plan_cluster(int M, int rows, int Gx, int bits, int group_size, bool whole_
   for (int s = 1; s <= (whole_tiles ? 1 : kCMaxSplit); ++s) {
     if (s > 1 && Gx < 4 * s) break;
     ClusterPlan c = {};
-    c.split = s; c.NT = NT; c.m_tiles = m_tiles; c.tiles = rows * m_tiles;
+    c.split = s; c.NT = NT; c.m_tiles = m_tiles; c.tiles = rows * m_tiles / unit;
     const int fit = max_clusters(s);
     if (fit < 1 || !cluster_layout(bits, group_size, &c)) continue;
     c.clusters = c.tiles < fit ? c.tiles : fit;
-    const int rounds = (c.tiles + c.clusters - 1) / c.clusters, len = (Gx + s - 1) / s;
+    const int rounds = unit * ((c.tiles + c.clusters - 1) / c.clusters), len = (Gx + s - 1) / s;
     double crowd = (c.clusters * s - sms / 2) / (s > 1 ? 0.27 * sms : 0.5 * sms);
     crowd = crowd < 0 ? 0 : (crowd > 1 ? 1 : crowd);
     const double cost = rounds * double(len) * kblock + 3.2 + (s > 1 ? 0.9 + 0.1 * s : 0.0) + 3.0 * crowd;
@@ -700,15 +728,24 @@ bool plan_cluster(int M, int rows, int Gx, int bits, int group_size, bool whole_
 
 }  // namespace
 
+long long gemm_wait_cycles() {
+  const char* e = getenv("B200LUT_WAIT_MS");
+  if (!e) return tc::kWaitCycles;
+  const long ms = atol(e);
+  return (ms < 1 ? 1 : ms > 1000 ? 1000 : ms) * 2000000ll;
+}
+
 bool cluster_gemm_serves(int M, int row_tiles, int K, int bits, int group_size) {
   ClusterPlan c = {};
-  return M >= 1 && group_size >= 64 && K >= 2 * kChunkK && plan_cluster(M, row_tiles, K / kChunkK, bits, group_size, true, &c);
+  return M >= 1 && group_size >= 64 && K >= 2 * kChunkK && plan_cluster(M, row_tiles, K / kChunkK, bits, group_size, true, 1, &c);
 }
 
 // `nseg` projections that share x (one code stream each, one code width and group size, at most two
-// palettes per 128-row tile); whole_tiles: K is not cut. *served is false, and nothing has been launched, for other shapes.
+// palettes per 128-row tile); whole_tiles: K is not cut; gated: the projections are (gate, up) of one
+// size, at most 16 rows, and segs[0].out becomes silu(gate) * up. *served is false, and nothing has been launched, for other shapes.
 int cluster_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b200lut_segment* segs, int nseg, bool pdl,
-                 void* stream, float* acc_out, const float* acc_in, long long ld_acc, long long wait_cycles, bool whole_tiles, bool* served) {
+                 void* stream, float* acc_out, const float* acc_in, long long ld_acc, long long wait_cycles, bool whole_tiles, bool gated,
+                 bool* served) {
   *served = false;
   ClusterParams p = {};
   int rows = 0, extra = 0;
@@ -738,11 +775,12 @@ int cluster_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b200
       if (blocks > extra) extra = blocks;
     }
   }
+  if (gated && (M > kCGatedMaxNT || nseg != 2 || segs[0].N != segs[1].N || extra || acc_out || acc_in)) return B200LUT_OK;
   p.nsegs = nseg;
   p.M = M; p.G = K / kChunkK; p.gs = segs[0].group_size;
   const int Gx = p.G + extra;
   ClusterPlan c = {};
-  if (segs[0].group_size < 64 || !plan_cluster(M, rows, Gx, segs[0].bits, p.gs, whole_tiles, &c)) return B200LUT_OK;
+  if (segs[0].group_size < 64 || !plan_cluster(M, rows, Gx, segs[0].bits, p.gs, whole_tiles, gated ? 2 : 1, &c)) return B200LUT_OK;
   p.NT = c.NT; p.m_tiles = c.m_tiles; p.split = c.split; p.clusters = c.clusters;
   p.tiles_each = c.tiles / c.clusters; p.tiles_more = c.tiles % c.clusters;
   p.kb_each = Gx / c.split; p.kb_more = Gx % c.split;
@@ -759,10 +797,13 @@ int cluster_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b200
     tmap = xmap;
   }
   *served = true;
-#define B200LUT_CLUSTER_AS(B, RES)                                                                          \
-  (dtype == B200LUT_BF16 ? launch_cluster<__nv_bfloat16, B, RES>(xmap, tmap, p, c.smem_bytes, pdl, cudaStream_t(stream)) \
-                         : launch_cluster<__half, B, RES>(xmap, tmap, p, c.smem_bytes, pdl, cudaStream_t(stream)))
-#define B200LUT_CLUSTER(B) (extra ? B200LUT_CLUSTER_AS(B, true) : B200LUT_CLUSTER_AS(B, false))
+#define B200LUT_CLUSTER_AS(B, MODE)                                                                         \
+  (dtype == B200LUT_BF16 ? launch_cluster<__nv_bfloat16, B, MODE>(xmap, tmap, p, c.smem_bytes, pdl, cudaStream_t(stream)) \
+                         : launch_cluster<__half, B, MODE>(xmap, tmap, p, c.smem_bytes, pdl, cudaStream_t(stream)))
+#define B200LUT_CLUSTER(B)                             \
+  (extra   ? B200LUT_CLUSTER_AS(B, kModeResidual)      \
+   : gated ? B200LUT_CLUSTER_AS(B, kModeGated)         \
+           : B200LUT_CLUSTER_AS(B, kModePlain))
   switch (segs[0].bits) {
     case 4: return B200LUT_CLUSTER(4);
     case 3: return B200LUT_CLUSTER(3);

@@ -1051,9 +1051,12 @@ extern "C" int b200lut_device_status(void) {
 namespace {
 constexpr int kClusterMaxM = 1024;
 constexpr long long kClusterMaxTiles = 640;
+// up to one token tile the cluster kernel is ahead at any number of row tiles (248320 x 4096: 147 us at
+// 32 tokens and 252 at 128, against 289 in the whole-tile kernel, which computes 256 columns in any case)
+constexpr int kClusterAnyM = 128;
 
 bool cluster_serves(int M, long long row_tiles, int K, int bits, int group_size) {
-  return M < kClusterMaxM && row_tiles * ((M + 127) / 128) <= kClusterMaxTiles && group_size >= 64 &&
+  return M < kClusterMaxM && (M <= kClusterAnyM || row_tiles * ((M + 127) / 128) <= kClusterMaxTiles) && group_size >= 64 &&
          cluster_gemm_serves(M, int(row_tiles), K, bits, group_size);
 }
 
@@ -1068,13 +1071,7 @@ int persistent_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b
   // heavy instrumentation can stretch a healthy wait beyond that; B200LUT_WAIT_MS raises the
   // bound for such runs (capped at one second).
   PersistParams pp = {};
-  pp.wait_cycles = tc::kWaitCycles;
-  if (const char* e = getenv("B200LUT_WAIT_MS")) {
-    long ms = atol(e);
-    if (ms < 1) ms = 1;
-    if (ms > 1000) ms = 1000;
-    pp.wait_cycles = (long long)ms * 2000000ll;
-  }
+  pp.wait_cycles = gemm_wait_cycles();
   const bool pdl = (flags & B200LUT_FLAG_PDL) != 0, cta_pairs = (flags & B200LUT_FLAG_CTA_PAIRS) != 0;
   {
     // Up to about four 128-token tiles per SM the cluster kernel is ahead (24576 x 4096: 24.7 against
@@ -1085,7 +1082,7 @@ int persistent_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b
     if (kg_rows == 0 && !(flags & B200LUT_FLAG_CTA_PAIRS) && cluster_serves(M, row_tiles, K, segs[0].bits, segs[0].group_size)) {
       bool served = false;
       const int rc = cluster_gemm(x, ldx, M, K, dtype, segs, nseg, pdl, stream, acc_out, acc_in, ld_acc, pp.wait_cycles,
-                                  (flags & B200LUT_FLAG_WHOLE_TILES) != 0, &served);
+                                  (flags & B200LUT_FLAG_WHOLE_TILES) != 0, false, &served);
       if (rc != B200LUT_OK || served) return rc;
     }
   }

@@ -827,6 +827,26 @@ bool rows_kernel_faster(const RowsGeom& g, int M) {
   return g.xreg || M < 2;
 }
 
+// Launches that the tensor-core kernel for batches (gemm_cluster.cu) takes over: from nine rows on, what
+// it serves (one code stream and no residual: that factor stays fp32 here, and would be rounded to 16
+// bits there). The tile kernel is ahead nowhere in that range: at 16 rows, per launch, tile kernel / here,
+// 4096 x 4096 10.1 / 6.8 us, 12288 x 4096 17.5 / 11.1 (3-bit 18.6 / 11.8), 4096 x 12288 16.2 / 13.4,
+// 1024 x 1024 7.8 / 3.7, 248320 x 4096 232 / 140; at nine rows 9.5 / 6.8, 16.7 / 11.1 (17.2 / 11.8),
+// 15.5 / 13.3, 6.9 / 3.9, 219 / 140. Up to eight rows the row-range kernel holds single launches of one
+// unit per block at best even (12288 x 4096 13.4 / 11.1 at eight) but a whole layer better.
+constexpr int kTensorCoreMinM = 9;
+
+bool tensor_core_decode(const GemvParams& p, int flags) {
+  if (p.M < kTensorCoreMinM || p.nseg > 4 || p.G < 2) return false;
+  if ((flags & (B200LUT_FLAG_TILE_KERNEL | B200LUT_FLAG_ROWS_KERNEL)) || !rows_kernel_wanted(0)) return false;
+  if (p.epilogue == B200LUT_EPI_SILU_MUL && p.nseg != 2) return false;
+  for (int i = 0; i < p.nseg; ++i) {
+    const SegDev& s = p.seg[i];
+    if (s.packed2 || s.res_rank || s.gs < 64 || s.bits != p.seg[0].bits || s.gs != p.seg[0].gs) return false;
+  }
+  return true;
+}
+
 // The layout of the row-range kernel for a launch, or false when the kernel does not serve it.
 // It depends only on the segment geometry; it is planned once per distinct launch shape (the
 // planner walks every 32-row unit) and looked up afterwards.
@@ -1137,6 +1157,12 @@ extern "C" int b200lut_gemv_input(const void* x, int64_t ldx, int M, int K, int 
   }
   const bool pdl = (flags & B200LUT_FLAG_PDL) != 0;
   cudaStream_t st = cudaStream_t(stream);
+  if (split <= 0 && !transformed && !p.ex.push && !p.ex.wait && tensor_core_decode(p, flags)) {
+    bool served = false;
+    const int rc = cluster_gemm(x, ldx, M, K, dtype, segs, nseg, pdl, stream, nullptr, nullptr, 0, gemm_wait_cycles(),
+                                false, silu, &served);
+    if (rc || served) return rc;
+  }
   // Library policy (split == 0): the row-range kernel when it serves the shapes. An explicit
   // split or B200LUT_FLAG_TILE_KERNEL selects the tile x split kernel.
   if (split <= 0 && rows_kernel_wanted(flags)) {

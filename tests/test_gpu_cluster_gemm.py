@@ -70,3 +70,49 @@ def test_merged_projections_with_and_without_a_residual():
     x = cases[0].x(M)
     want = torch.cat([c.oracle(x) for c in cases], dim=-1)
     assert rel_err(qkv(x.cuda()), want) <= TOL
+
+
+@pytest.mark.parametrize("N,K,gs,bits,dtype,M,bias", (
+    (128, 128, 128, 4, torch.bfloat16, 9, False),                      # the fewest k-blocks
+    (256, 4160, 128, 4, torch.float16, 16, True),                      # eight CTAs share four token quads
+    (384, 1984, 64, 3, torch.bfloat16, 13, True),
+    (128, 832, 256, 2, torch.float16, 12, False),
+    (256, 1088, 512, 1, torch.bfloat16, 16, True),
+    (19200, 192, 128, 4, torch.bfloat16, 10, False),                   # 150 row tiles
+))
+def test_batched_decode(N, K, gs, bits, dtype, M, bias):
+    case = Case(N, K, gs, bits, dtype, seed=N + K + M, bias=bias)
+    x = case.x(M)
+    got = case.module()(x.cuda())
+    assert rel_err(got, case.oracle(x)) <= TOL
+
+
+@pytest.mark.parametrize("N,K,gs,bits,dtype,M,aligned", (
+    (128, 128, 128, 4, torch.bfloat16, 9, True),
+    (256, 4160, 64, 4, torch.float16, 16, False),                      # a cut over eight CTAs, two palettes, odd stride
+    (384, 1984, 128, 3, torch.bfloat16, 11, True),
+    (19328, 128, 128, 2, torch.float16, 16, True),                     # 151 pairs of tiles
+))
+def test_batched_gated_pair(N, K, gs, bits, dtype, M, aligned):
+    gate, up = (Case(N, K, gs, bits, dtype, seed=7 * N + K + i, bias=(i == 0)) for i in range(2))
+    x = gate.x(M)
+    mods = [gate.module(), up.module()]
+    ld = N if aligned else N + 3
+    out = torch.full((M, ld), float("nan"), dtype=dtype, device="cuda")
+    descs = []
+    for m in mods:
+        m._ensure_packed()
+        descs.append(dict(packed=m._packed, lut=m.lut, N=N, group_size=gs, n_groups=m.lut.shape[0], bits=bits,
+                          bias=m.bias, out=out, ldo=ld))
+    L.gemv_multi(x.cuda(), L.make_segments(descs), 2, epilogue=L.EPI_SILU_MUL)
+    g, u = (torch.nn.functional.linear(x.double(), c.w1.double(), None if c.bias is None else c.bias.double()) for c in (gate, up))
+    want = torch.nn.functional.silu(g) * u                             # fp32 sums, one rounding: 2^-8 of a value in bf16
+    assert rel_err(out[:, :N], want.float()) <= 2.0 ** -8
+    assert torch.isnan(out[:, N:].float()).all()
+
+
+@pytest.mark.parametrize("M", (20, 128))
+def test_more_row_tiles_than_the_token_tiles_pay_for(M):
+    case = Case(128 * 700, 128, 128, 4, torch.bfloat16, seed=M)        # 700 row tiles
+    x = case.x(M)
+    assert rel_err(case.module()(x.cuda()), case.oracle(x)) <= TOL
