@@ -288,7 +288,7 @@ typedef struct b200lut_exchange {
  * segments with split = 0 (the library's policy) — the producer_blocks of an exchange whose
  * pushing launch they describe. Output pointers of the segments may be NULL here. 0 on invalid
  * arguments. The policy picks between the two decode kernels by shape and M (a launch without an
- * exchange may run the tensor-core kernel from nine rows on, which has no exchange); a launch that
+ * exchange may run the tensor-core kernel from three rows on, which has no exchange); a launch that
  * carries an input transform or a flag-less (sentinel) exchange always runs the row-range
  * kernel, so pass B200LUT_FLAG_ROWS_KERNEL here for such a launch. No counterpart in the
  * reference. */

@@ -1,4 +1,4 @@
-// LUT GEMM for batches of 9 to a few hundred rows (batched decode, short prompts) on tcgen05.
+// LUT GEMM for batches of 3 to a few hundred rows (batched decode, short prompts) on tcgen05.
 //
 // Such a launch is a stream of codes with little arithmetic per code: at 64 rows a 128 x 64 chunk of
 // 4-bit codes (4 KB of HBM, 177 cycles of an SM's share) feeds four MMAs of 128 x 64 x 16 (149
@@ -701,7 +701,12 @@ int max_clusters(int split) {
 // The cut of K that finishes first, by a fit (microseconds) to launches measured at 2048 to 24576 rows,
 // K = 4096 and 12288, 24 to 1024 tokens, cuts of 1 to 8: a k-block of the busiest cluster, what a launch
 // costs besides, what the exchange adds, and what is lost when the launch fills more than half of the
-// SMs (below that, its start and end run beside its neighbours' in the stream). `unit` tiles go to a
+// SMs (below that, its start and end run beside its neighbours' in the stream). With K cut, a cluster's
+// next tile cannot end before the exchange of the last one has made its way around (kExchange: 16 rows of
+// 24576 x 4096, a gate/up pair, cuts of 1 / 2 / 3 / 8 over 2 / 4 / 4 to 6 / 12 tiles, 20.5 / 23.2 / 32.2 /
+// 57.7 us): short parts of many tiles lose what the even split gains. With that term in the cost the pair
+// takes 20.7 us instead of 30.9, 248320 x 4096 at 16 rows 125 instead of 144, and the Q/K/V launch of 333
+// tokens and its residual 53 instead of 84. `unit` tiles go to a
 // cluster together; c.tiles counts units.
 bool plan_cluster(int M, int rows, int Gx, int bits, int group_size, bool whole_tiles, int unit, ClusterPlan* best) {
   const int m_tiles = (M + kCMaxNT - 1) / kCMaxNT;
@@ -710,6 +715,7 @@ bool plan_cluster(int M, int rows, int Gx, int bits, int group_size, bool whole_
   const double kblock = 0.112 + 4.7e-6 * NT * NT;
   double least = 0;
   bool found = false;
+  constexpr double kExchange = 3.9;
   for (int s = 1; s <= (whole_tiles ? 1 : kCMaxSplit); ++s) {
     if (s > 1 && Gx < 4 * s) break;
     ClusterPlan c = {};
@@ -720,7 +726,8 @@ bool plan_cluster(int M, int rows, int Gx, int bits, int group_size, bool whole_
     const int rounds = unit * ((c.tiles + c.clusters - 1) / c.clusters), len = (Gx + s - 1) / s;
     double crowd = (c.clusters * s - sms / 2) / (s > 1 ? 0.27 * sms : 0.5 * sms);
     crowd = crowd < 0 ? 0 : (crowd > 1 ? 1 : crowd);
-    const double cost = rounds * double(len) * kblock + 3.2 + (s > 1 ? 0.9 + 0.1 * s : 0.0) + 3.0 * crowd;
+    const double tile = double(len) * kblock, next = s > 1 && tile < kExchange ? kExchange : tile;
+    const double cost = tile + (rounds - 1) * next + 3.2 + (s > 1 ? 0.9 + 0.1 * s : 0.0) + 3.0 * crowd;
     if (!found || cost < least) { *best = c; least = cost; found = true; }
   }
   return found;

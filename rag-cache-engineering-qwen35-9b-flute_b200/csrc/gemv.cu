@@ -827,17 +827,23 @@ bool rows_kernel_faster(const RowsGeom& g, int M) {
   return g.xreg || M < 2;
 }
 
-// Launches that the tensor-core kernel for batches (gemm_cluster.cu) takes over: from nine rows on, what
-// it serves (one code stream and no residual: that factor stays fp32 here, and would be rounded to 16
-// bits there). The tile kernel is ahead nowhere in that range: at 16 rows, per launch, tile kernel / here,
-// 4096 x 4096 10.1 / 6.8 us, 12288 x 4096 17.5 / 11.1 (3-bit 18.6 / 11.8), 4096 x 12288 16.2 / 13.4,
-// 1024 x 1024 7.8 / 3.7, 248320 x 4096 232 / 140; at nine rows 9.5 / 6.8, 16.7 / 11.1 (17.2 / 11.8),
-// 15.5 / 13.3, 6.9 / 3.9, 219 / 140. Up to eight rows the row-range kernel holds single launches of one
-// unit per block at best even (12288 x 4096 13.4 / 11.1 at eight) but a whole layer better.
-constexpr int kTensorCoreMinM = 9;
+// Launches that the tensor-core kernel for batches (gemm_cluster.cu) takes over, of those it serves: one
+// code stream and no residual (that factor stays fp32 here, and would be rounded to 16 bits there). Its
+// time does not depend on the rows up to 16; us here / there:
+//  * from nine rows on it is ahead everywhere (at 9 rows 4096 x 4096 9.5 / 6.8, 12288 x 4096 16.7 / 11.1,
+//    3-bit 17.2 / 11.8, 4096 x 12288 15.5 / 13.3, 1024 x 1024 6.9 / 3.9, 248320 x 4096 219 / 125; eight
+//    captured decoder layers 605 / 442);
+//  * from three rows on a launch of many row tiles per SM gains (3 rows: 128000 x 4096 75.5 / 65.5,
+//    248320 x 4096 141 / 125); at two it does not (118 / 124).
+// A step of five to eight rows would gain as well (layers 496 / 442 at five, 519 / 441 at eight), but there
+// a projection's plain launch has the bits of its launch with an exchange, with the transform inside or
+// in a persistent plan, which all run the row-range kernel.
+constexpr int kTensorCoreMinM = 9, kTensorCoreMinMHead = 3;
+constexpr int kTensorCoreHeadTiles = 1000;
 
 bool tensor_core_decode(const GemvParams& p, int flags) {
-  if (p.M < kTensorCoreMinM || p.nseg > 4 || p.G < 2) return false;
+  const int min_m = p.seg[0].bits == 4 && p.tiles_total >= kTensorCoreHeadTiles ? kTensorCoreMinMHead : kTensorCoreMinM;
+  if (p.M < min_m || p.nseg > 4 || p.G < 2) return false;
   if ((flags & (B200LUT_FLAG_TILE_KERNEL | B200LUT_FLAG_ROWS_KERNEL)) || !rows_kernel_wanted(0)) return false;
   if (p.epilogue == B200LUT_EPI_SILU_MUL && p.nseg != 2) return false;
   for (int i = 0; i < p.nseg; ++i) {

@@ -79,6 +79,7 @@ def test_merged_projections_with_and_without_a_residual():
     (128, 832, 256, 2, torch.float16, 12, False),
     (256, 1088, 512, 1, torch.bfloat16, 16, True),
     (19200, 192, 128, 4, torch.bfloat16, 10, False),                   # 150 row tiles
+    (128 * 1000, 128, 128, 4, torch.bfloat16, 3, False),               # the fewest rows of many row tiles
 ))
 def test_batched_decode(N, K, gs, bits, dtype, M, bias):
     case = Case(N, K, gs, bits, dtype, seed=N + K + M, bias=bias)
