@@ -430,6 +430,9 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
     // Token quads (four columns): CTA r of the cluster finishes quads [first(r), first(r + 1)).
     auto first = [&](int r) { return r * p.quads_each + (r < p.quads_more ? r : p.quads_more); };
     const int mine0 = first(rank), mine1 = first(rank + 1);
+    // Has this warp quads of its half to send? Where no other CTA's share is wider than two quads, the warps of
+    // the second half have none, and nobody waits for them: the exchange may be a tile or two ahead of them.
+    const bool sends = p.quads_each + (p.quads_more > (rank < p.quads_more ? 1 : 0) ? 1 : 0) > 2 * h;
     uint32_t e_quad = p.e_quad;
     pin(e_quad);
     const uint32_t slot_stride = uint32_t(p.quads_each + (p.quads_more ? 1 : 0)) * e_quad;   // of the widest share
@@ -455,7 +458,10 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
       tc::mbar_wait(bar_dfull + 8 * (t & 1), uint32_t(t >> 1) & 1u, abort_flag, &g_cluster_status, tc::kStatusWaitDone, lim);
       tc::fence_after_sync();
       if (S > 1) {
-        if (t > 0)     // the others have read this CTA's parts of the last tile
+        // The others have read this CTA's parts of the last tile. A warp that sends nothing overwrites nothing,
+        // and must not wait here: the phase it asks for could be two back, which reads as not complete.
+        // A warp that sends cannot miss one, as the next phase needs what it sends.
+        if (t > 0 && sends)
           tc::mbar_wait_cluster(bar_efree, uint32_t(t - 1) & 1u, abort_flag, &g_cluster_status, tc::kStatusWaitDone, lim);
         for (int k = 1; k < S; ++k) {
           const int d = rank + k < S ? rank + k : rank + k - S;

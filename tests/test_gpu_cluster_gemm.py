@@ -1,7 +1,7 @@
 """The tensor-core GEMM for batches and short prompts (csrc/gemm_cluster.cu) where it can go wrong: token
-counts at the edges of its 16- to 128-token tiles, odd and few k-blocks per CTA, every cut of K its
-planner picks (few row tiles: up to eight CTAs per cluster), two palettes per tile, every code width,
-merged projections, residual k-blocks that start in the middle of a stage, unaligned outputs."""
+counts at the edges of its 16- to 128-token tiles, odd and few k-blocks per CTA, cuts of K over up to eight
+CTAs per cluster with one tile each and with several one after the other, two palettes per tile, every code
+width, merged projections, residual k-blocks that start in the middle of a stage, unaligned outputs."""
 from __future__ import annotations
 
 import pytest
@@ -117,3 +117,42 @@ def test_more_row_tiles_than_the_token_tiles_pay_for(M):
     case = Case(128 * 700, 128, 128, 4, torch.bfloat16, seed=M)        # 700 row tiles
     x = case.x(M)
     assert rel_err(case.module()(x.cuda()), case.oracle(x)) <= TOL
+
+
+def _synthetic(N, K, bits, gs, dtype=torch.float16, seed=0):
+    g = torch.Generator().manual_seed(N + K + seed)
+    blob = pkg.synthetic.random_blob_on_device(N, K, bits, N + K + seed, "cuda")
+    lut = (0.02 * torch.randn(-(-N // gs), 1 << bits, generator=g)).sort(dim=1).values.to(dtype).cuda()
+    return pkg.PalettizedLinear(blob, lut, bits, gs, N, K)
+
+
+@pytest.mark.parametrize("N,K,bits,M,dtype", (                         # on 148 SMs:
+    (19200, 4096, 4, 9, torch.bfloat16),                               # cut 2, three tiles per cluster
+    (19200, 6144, 3, 16, torch.float16),                               # cut 3, four tiles; one or two token quads per CTA
+    (12800, 12288, 4, 17, torch.bfloat16),                             # cut 5, four tiles
+    (19200, 12288, 4, 64, torch.bfloat16),                             # cut 6, seven tiles
+    (11776, 6144, 2, 128, torch.float16),                              # cut 4, three full tiles
+))
+def test_cut_tiles_one_after_the_other(N, K, bits, M, dtype):
+    # the exchange's barriers change phase with every tile of a cluster, the accumulators with every other one
+    mod = _synthetic(N, K, bits, 128, dtype)
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(dtype).cuda()
+    got = mod(x)
+    want = x.double() @ (mod._quantized_weight().double()).t()
+    assert rel_err(got, want.float()) <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)   # one rounding
+    for _ in range(20):
+        assert torch.equal(mod(x), got)
+
+
+@pytest.mark.parametrize("N,M", ((6400, 9), (12800, 16)))
+def test_cut_gated_tiles_one_after_the_other(N, M):
+    K, dt = 12288, torch.bfloat16                                      # cut 5: four and eight tiles per cluster
+    mods = [_synthetic(N, K, 4, 128, dt, seed=i) for i in range(2)]
+    x = (0.1 * torch.randn(M, K, generator=torch.Generator().manual_seed(M))).to(dt).cuda()
+    out = torch.empty(M, N, dtype=dt, device="cuda")
+    segs = L.make_segments([m._segment_desc(out) for m in mods])
+    g, u = (x.double() @ m._quantized_weight().double().t() for m in mods)
+    for _ in range(20):
+        out.fill_(float("nan"))
+        L.gemv_multi(x, segs, 2, epilogue=L.EPI_SILU_MUL)
+        assert rel_err(out, (torch.nn.functional.silu(g) * u).float()) <= 2.0 ** -8
