@@ -94,12 +94,13 @@ int exchange_status_take();
 // Status word of the batched-decode tensor-core GEMM: value and clear.
 int gemm_cluster_status_take();
 // That GEMM (gemm_cluster.cu); *served is false, and nothing has been launched, for shapes it does not take.
+// chain_limit: k-blocks of 64 columns that one tensor-core accumulator may sum, whose error grows with them.
 int cluster_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b200lut_segment* segs, int nseg, bool pdl,
                  void* stream, float* acc_out, const float* acc_in, long long ld_acc, long long wait_cycles, bool whole_tiles, bool gated,
-                 bool* served);
+                 int chain_limit, bool* served);
 // The bound of the tensor-core kernels' in-kernel waits, in SM clock cycles (B200LUT_WAIT_MS raises it).
 long long gemm_wait_cycles();
-bool cluster_gemm_serves(int M, int row_tiles, int K, int bits, int group_size);
+bool cluster_gemm_serves(int M, int row_tiles, int K, int bits, int group_size, int chain_limit);
 // Status word of the embedding gather (an id outside the table): value and clear.
 int embed_status_take();
 

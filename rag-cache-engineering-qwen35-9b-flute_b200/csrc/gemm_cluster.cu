@@ -16,8 +16,16 @@
 //    distributed shared memory (each finishes a share of the tokens, adding the parts in ascending-k
 //    order), so a 4096-row projection fills the GPU without a workspace, and tiles that do not divide
 //    by the SM count cost less.
-//  * Two accumulators, and eight epilogue warps of their own: a tile's exchange and stores run under
+//  * Two accumulator halves, and eight epilogue warps of their own: a tile's exchange and stores run under
 //    the next tile's MMAs.
+//  * Sums in chains: the tensor core truncates where it adds to its fp32 accumulator, so a sum's error
+//    grows with the number of MMAs behind one another (share of fp16 results that are not the rounding of
+//    the 64-bit sum, K = 4096: 1.72e-2 for one chain, 0.95e-2 for two, 0.52e-2 for four). A tile's
+//    k-blocks therefore go to several accumulators one after the other, which the epilogue adds in fp32,
+//    ascending: as many as keep every chain as short as in the kernel that would serve the launch
+//    otherwise (`chain_limit`: the tile kernel's warps at up to 16 rows, the cut tiles of gemm_tc.cu
+//    above). Where they do not fit into half of the columns, a tile takes both halves and the next tile's
+//    MMAs start when they have been read.
 // Weights are the A operand in tensor memory, tokens (up to 128 per tile) the B operand in shared
 // memory, as in gemm_tc.cu. All waits are bounded.
 //
@@ -70,6 +78,7 @@ struct ClusterParams {
   int kb_each, kb_more;                          // k-blocks per CTA of a cluster, CTAs (the first ones) with one more
   int quads_each, quads_more;                    // token quads that a CTA finishes, likewise
   int NT, m_tiles, G, gs, M, nx, nc;             // tokens per tile, token tiles, ..., activation slots, code slots
+  int chain, halves;                             // k-blocks per accumulator (1 or even); 2: tiles alternate between the halves
   uint32_t slot_bytes, x_off, c_off, e_off, s_off;   // offsets inside the shared window
   uint32_t e_quad, e_rows8;                          // exchange slots: bytes from quad to quad, from eight rows to the next eight
   int nsegs;
@@ -402,24 +411,34 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
       uint32_t half = uint32_t(p.NT) * 8u;                  // one k-block of activations in descriptor units
       int nx = p.nx, slot = 0;
       pin(half); pin(nx);
-      uint32_t st = 0, acc = tmem, xlo = x0;
+      const int alt = p.halves - 1;                         // 1: tile t in half t & 1
+      uint32_t st = 0, xlo = x0;
+      // A chain's first k-block overwrites its accumulator. Chains are whole stages, or single k-blocks: then
+      // the stage's second one has the next accumulator. (Loop-invariant values and a count: with the chains
+      // in a loop of their own 12288 x 4096, 3 bits, 16 rows took 13.0 instead of 12.4 us.)
+      const bool one = p.chain == 1;
+      const uint32_t next = half >> 3, next_half = one ? next : 0u, add_half = one ? 0u : 1u, jump = next + next_half;
       for (int t = 0; t < ntile; ++t) {
-        if (t >= 2)                    // the accumulator's last tile must have been read
-          tc::mbar_wait(bar_dempty + 8 * (t & 1), uint32_t((t >> 1) - 1) & 1u, abort_flag, &g_cluster_status,
+        const int buf = t & alt;
+        if (t > alt)                   // the half's last tile must have been read
+          tc::mbar_wait(bar_dempty + 8 * buf, uint32_t((t >> alt) - 1) & 1u, abort_flag, &g_cluster_status,
                         tc::kStatusWaitDone, lim);
+        uint32_t acc = tmem + uint32_t(buf * kCMaxNT), add = 0u;
+        int left = p.chain;
         for (int j = 0; j < lp; j += 2, ++st) {
           const uint32_t u = st & (kCStages - 1);
           const bool second = !RES || j < pc ? j + 1 < lenc : j - pc + 1 < lenr;
           tc::mbar_wait(bar_full + 8 * u, (st / kCStages) & 1u, abort_flag, &g_cluster_status, tc::kStatusWaitFull, lim);
           tc::fence_after_sync();
-          tc::mma_ts_kblock(acc, tmem + kCACol + 64u * u, xlo, xhi, idesc, j == 0 ? 0u : 1u);
-          if (second) tc::mma_ts_kblock(acc, tmem + kCACol + 64u * u + 32u, xlo + half, xhi, idesc, 1u);
+          tc::mma_ts_kblock(acc, tmem + kCACol + 64u * u, xlo, xhi, idesc, add);
+          if (second) tc::mma_ts_kblock(acc + next_half, tmem + kCACol + 64u * u + 32u, xlo + half, xhi, idesc, add_half);
           tc::mma_commit(bar_done + 8 * u);
+          add = 1u;
+          if ((left -= 2) <= 0) { left = p.chain; acc += jump; add = 0u; }
           xlo += 2 * half;
           if (++slot == nx) { slot = 0; xlo = x0; }
         }
-        tc::mma_commit(bar_dfull + 8 * (t & 1));
-        acc ^= uint32_t(kCMaxNT);
+        tc::mma_commit(bar_dfull + 8 * buf);
       }
     }
     __syncwarp();
@@ -438,9 +457,32 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
     const uint32_t slot_stride = uint32_t(p.quads_each + (p.quads_more ? 1 : 0)) * e_quad;   // of the widest share
     const uint32_t exch = win + p.e_off + uint32_t(row_in >> 3) * p.e_rows8 + uint32_t(row_in & 7) * 16u;
     const uint32_t stage = win + p.s_off + uint32_t(warp - kCEpiWarp) * 512u;   // 8 tokens x 32 rows
+    const int alt = p.halves - 1;
+    // accumulators of this CTA's tiles (the residual's k-blocks start a stage of their own),
+    int chains = (p.chain == 1 ? len : lp + p.chain - 1) / p.chain;
+    const uint32_t chain_cols = uint32_t(p.NT);                    // and the columns from one to the next
+    pin(chains);
+    // Quads b and, with `both`, b + 1 of the accumulators at `acc`: their chains' sums, ascending in k.
+    auto read_quads = [&](uint32_t acc, int b, bool both, uint32_t (&r)[2][4]) {
+      const uint32_t a = acc + uint32_t(4 * b);
+      tmem_ld_32x32b_x4(a, r[0]);
+      if (both) tmem_ld_32x32b_x4(a + 4u, r[1]);
+      tc::wait_ld();
+#pragma unroll 1
+      for (int i = 1; i < chains; ++i) {
+        uint32_t u[2][4];
+        tmem_ld_32x32b_x4(a + uint32_t(i) * chain_cols, u[0]);
+        if (both) tmem_ld_32x32b_x4(a + uint32_t(i) * chain_cols + 4u, u[1]);
+        tc::wait_ld();
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (e == 0 || both) r[e][j] = __float_as_uint(__uint_as_float(r[e][j]) + __uint_as_float(u[e][j]));
+      }
+    };
     float* acc_out = p.acc_out;
     const float* acc_in = p.acc_in;
-    pin(acc_out); pin(acc_in);
     float gate[8];                                                 // gated form: what the last (gate) tile came to
     for (int t = 0; t < ntile; ++t) {
       const int row = row_of(t0 + t), m0 = tok_of(t0 + t);
@@ -452,10 +494,16 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
       pin(out); pin(ldo); pin(M);
       const bool vec = (GATED ? p.seg[0].out_aligned : sd.out_aligned) != 0;
       const float bias = sd.bias ? DType<T>::to_float(sd.bias[n + lane]) : 0.f;
-      const uint32_t acc = tmem + (uint32_t(32 * q) << 16) + uint32_t(t & 1) * kCMaxNT;
+      const int buf = t & alt;
+      const uint32_t acc = tmem + (uint32_t(32 * q) << 16) + uint32_t(buf * kCMaxNT);
+      auto release = [&]() {                                       // this warp has read the tile's accumulators
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(bar_dempty + 8 * buf);
+      };
       if (S > 1 && warp == kCEpiWarp && lane == 0)                 // what the others will write here for this tile
         tc::mbar_expect_tx(bar_efull, uint32_t((S - 1) * (mine1 - mine0) * kTileRows) * 16u);
-      tc::mbar_wait(bar_dfull + 8 * (t & 1), uint32_t(t >> 1) & 1u, abort_flag, &g_cluster_status, tc::kStatusWaitDone, lim);
+      tc::mbar_wait(bar_dfull + 8 * buf, uint32_t(t >> alt) & 1u, abort_flag, &g_cluster_status, tc::kStatusWaitDone, lim);
       tc::fence_after_sync();
       if (S > 1) {
         // The others have read this CTA's parts of the last tile. A warp that sends nothing overwrites nothing,
@@ -471,22 +519,20 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
           uint32_t dst = map_rank(exch, uint32_t(d)) + uint32_t(rank < d ? rank : rank - 1) * slot_stride +
                          uint32_t(2 * h) * e_quad;
           for (int b = b0 + 2 * h; b < b1; b += 4, dst += 4u * e_quad) {
-            uint32_t r0[4], r1[4];
-            tmem_ld_32x32b_x4(acc + uint32_t(4 * b), r0);
-            if (b + 1 < b1) tmem_ld_32x32b_x4(acc + uint32_t(4 * b + 4), r1);
-            tc::wait_ld();
-            st_async_v4(dst, bar, r0);
-            if (b + 1 < b1) st_async_v4(dst + e_quad, bar, r1);
+            uint32_t r[2][4];
+            read_quads(acc, b, b + 1 < b1, r);
+            st_async_v4(dst, bar, r[0]);
+            if (b + 1 < b1) st_async_v4(dst + e_quad, bar, r[1]);
           }
         }
         tc::mbar_wait_cluster(bar_efull, uint32_t(t) & 1u, abort_flag, &g_cluster_status, tc::kStatusWaitFull, lim);
       }
+      if (mine0 + 2 * h >= mine1) release();
       for (int b = mine0 + 2 * h; b < mine1; b += 4) {             // 8 tokens of the warp's 32 rows at a time
         const bool both = b + 1 < mine1;
         uint32_t own[2][4];
-        tmem_ld_32x32b_x4(acc + uint32_t(4 * b), own[0]);
-        if (both) tmem_ld_32x32b_x4(acc + uint32_t(4 * b + 4), own[1]);
-        tc::wait_ld();
+        read_quads(acc, b, both, own);
+        if (b + 4 >= mine1) release();
         float v[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = S == 1 ? __uint_as_float(own[j >> 2][j & 3]) : 0.f;
@@ -550,9 +596,6 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
             if (j < ntok) out[(tok0 + j) * ldo + lane] = DType<T>::from_float(GATED ? v[j] : v[j] + bias);
         }
       }
-      tc::fence_before_sync();
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(bar_dempty + 8 * (t & 1));
       if (S > 1 && t + 1 < ntile) {
         asm volatile("fence.acq_rel.cluster;" ::: "memory");
         __syncwarp();
@@ -578,7 +621,7 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
 // ---- host -------------------------------------------------------------------------------------------
 
 struct ClusterPlan {
-  int split, clusters, NT, m_tiles, tiles, nx, nc;
+  int split, clusters, NT, m_tiles, tiles, nx, nc, chains, chain, halves;
   uint32_t slot_bytes, x_off, c_off, e_off, s_off, e_quad, e_rows8, smem_bytes;
 };
 
@@ -711,29 +754,41 @@ int max_clusters(int split) {
 // next tile cannot end before the exchange of the last one has made its way around (kExchange: 16 rows of
 // 24576 x 4096, a gate/up pair, cuts of 1 / 2 / 3 / 8 over 2 / 4 / 4 to 6 / 12 tiles, 20.5 / 23.2 / 32.2 /
 // 57.7 us): short parts of many tiles lose what the even split gains. With that term in the cost the pair
-// takes 20.7 us instead of 30.9, 248320 x 4096 at 16 rows 125 instead of 144, and the Q/K/V launch of 333
+// takes 20.7 us instead of 30.9, 248320 x 4096 at 16 rows 126 instead of 144, and the Q/K/V launch of 333
 // tokens and its residual 53 instead of 84. `unit` tiles go to a
-// cluster together; c.tiles counts units.
-bool plan_cluster(int M, int rows, int Gx, int bits, int group_size, bool whole_tiles, int unit, ClusterPlan* best) {
+// cluster together; c.tiles counts units. `chain_limit`: the most of the G k-blocks that one accumulator may
+// take; a cut whose chains do not fit into the accumulators' columns is out. (The residual's `extra` k-blocks
+// lengthen a chain, as they do in the kernel the limit comes from.)
+bool plan_cluster(int M, int rows, int G, int extra, int bits, int group_size, bool whole_tiles, int unit, int chain_limit,
+                  ClusterPlan* best) {
+  const int Gx = G + extra;
   const int m_tiles = (M + kCMaxNT - 1) / kCMaxNT;
   const int per = (M + m_tiles - 1) / m_tiles, NT = (per + 15) / 16 * 16;
   const int sms = max_clusters(1);
   const double kblock = 0.112 + 4.7e-6 * NT * NT;
   double least = 0;
   bool found = false;
-  constexpr double kExchange = 3.9;
+  constexpr double kExchange = 3.9, kDrain = 0.5;
   for (int s = 1; s <= (whole_tiles ? 1 : kCMaxSplit); ++s) {
     if (s > 1 && Gx < 4 * s) break;
     ClusterPlan c = {};
     c.split = s; c.NT = NT; c.m_tiles = m_tiles; c.tiles = rows * m_tiles / unit;
+    // chains of whole stages (two k-blocks), or of single k-blocks; the residual's start a stage of their own
+    const int len = (Gx + s - 1) / s, coded = (G + s - 1) / s;
+    const int limit = chain_limit >= coded ? (coded + 1) & ~1 : chain_limit > 1 ? chain_limit & ~1 : 1;
+    c.chains = limit == 1 ? len : (coded + limit - 1) / limit;
+    c.chain = limit == 1 ? 1 : (((len + (extra ? 2 : 0) + c.chains - 1) / c.chains) + 1) & ~1;
+    if (c.chains * NT > 2 * kCMaxNT) continue;
+    c.halves = c.chains * NT > kCMaxNT ? 1 : 2;
     const int fit = max_clusters(s);
     if (fit < 1 || !cluster_layout(bits, group_size, &c)) continue;
     c.clusters = c.tiles < fit ? c.tiles : fit;
-    const int rounds = unit * ((c.tiles + c.clusters - 1) / c.clusters), len = (Gx + s - 1) / s;
+    const int rounds = unit * ((c.tiles + c.clusters - 1) / c.clusters);
     double crowd = (c.clusters * s - sms / 2) / (s > 1 ? 0.27 * sms : 0.5 * sms);
     crowd = crowd < 0 ? 0 : (crowd > 1 ? 1 : crowd);
     const double tile = double(len) * kblock, next = s > 1 && tile < kExchange ? kExchange : tile;
-    const double cost = tile + (rounds - 1) * next + 3.2 + (s > 1 ? 0.9 + 0.1 * s : 0.0) + 3.0 * crowd;
+    const double cost = tile + (rounds - 1) * (next + (c.halves == 1 ? kDrain : 0.0)) + 3.2 +
+                        (s > 1 ? 0.9 + 0.1 * s : 0.0) + 3.0 * crowd;
     if (!found || cost < least) { *best = c; least = cost; found = true; }
   }
   return found;
@@ -748,9 +803,10 @@ long long gemm_wait_cycles() {
   return (ms < 1 ? 1 : ms > 1000 ? 1000 : ms) * 2000000ll;
 }
 
-bool cluster_gemm_serves(int M, int row_tiles, int K, int bits, int group_size) {
+bool cluster_gemm_serves(int M, int row_tiles, int K, int bits, int group_size, int chain_limit) {
   ClusterPlan c = {};
-  return M >= 1 && group_size >= 64 && K >= 2 * kChunkK && plan_cluster(M, row_tiles, K / kChunkK, bits, group_size, true, 1, &c);
+  return M >= 1 && group_size >= 64 && K >= 2 * kChunkK &&
+         plan_cluster(M, row_tiles, K / kChunkK, 0, bits, group_size, false, 1, chain_limit, &c);
 }
 
 // `nseg` projections that share x (one code stream each, one code width and group size, at most two
@@ -758,7 +814,7 @@ bool cluster_gemm_serves(int M, int row_tiles, int K, int bits, int group_size) 
 // size, at most 16 rows, and segs[0].out becomes silu(gate) * up. *served is false, and nothing has been launched, for other shapes.
 int cluster_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b200lut_segment* segs, int nseg, bool pdl,
                  void* stream, float* acc_out, const float* acc_in, long long ld_acc, long long wait_cycles, bool whole_tiles, bool gated,
-                 bool* served) {
+                 int chain_limit, bool* served) {
   *served = false;
   ClusterParams p = {};
   int rows = 0, extra = 0;
@@ -793,10 +849,13 @@ int cluster_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b200
   p.M = M; p.G = K / kChunkK; p.gs = segs[0].group_size;
   const int Gx = p.G + extra;
   ClusterPlan c = {};
-  if (segs[0].group_size < 64 || !plan_cluster(M, rows, Gx, segs[0].bits, p.gs, whole_tiles, gated ? 2 : 1, &c)) return B200LUT_OK;
+  if (segs[0].group_size < 64 ||
+      !plan_cluster(M, rows, p.G, extra, segs[0].bits, p.gs, whole_tiles, gated ? 2 : 1, whole_tiles ? p.G : chain_limit, &c))
+    return B200LUT_OK;
   p.NT = c.NT; p.m_tiles = c.m_tiles; p.split = c.split; p.clusters = c.clusters;
   p.tiles_each = c.tiles / c.clusters; p.tiles_more = c.tiles % c.clusters;
   p.kb_each = Gx / c.split; p.kb_more = Gx % c.split;
+  p.halves = c.halves; p.chain = c.chain;
   p.quads_each = c.NT / 4 / c.split; p.quads_more = c.NT / 4 % c.split;
   p.nx = c.nx; p.nc = c.nc; p.slot_bytes = c.slot_bytes;
   p.x_off = c.x_off; p.c_off = c.c_off; p.e_off = c.e_off; p.s_off = c.s_off; p.e_quad = c.e_quad; p.e_rows8 = c.e_rows8;

@@ -1051,13 +1051,30 @@ extern "C" int b200lut_device_status(void) {
 namespace {
 constexpr int kClusterMaxM = 1024;
 constexpr long long kClusterMaxTiles = 640;
-// up to one token tile the cluster kernel is ahead at any number of row tiles (248320 x 4096: 147 us at
-// 32 tokens and 252 at 128, against 289 in the whole-tile kernel, which computes 256 columns in any case)
+// up to one token tile the cluster kernel is ahead at any number of row tiles (248320 x 4096: 132 us at
+// 32 tokens and 249 at 128, against 289 in the whole-tile kernel, which computes 256 columns in any case)
 constexpr int kClusterAnyM = 128;
 
-bool cluster_serves(int M, long long row_tiles, int K, int bits, int group_size) {
+long long persistent_tiles(int M, long long row_tiles) {
+  const int nt = M >= kPMaxNT ? kPMaxNT : ((M + 31) / 32) * 32;
+  return row_tiles * ((M + nt - 1) / nt);
+}
+
+// k-blocks that one accumulator of the persistent kernel sums in such a launch: all of them in a whole tile,
+// a part of them in the tiles of the last round, which are cut; their mean, since the cluster kernel cuts
+// every tile alike.
+int persistent_chain(int M, long long row_tiles, int G, int sms) {
+  const long long tiles = persistent_tiles(M, row_tiles);
+  const SplitPlan sp = plan_split(tiles, G, sms);
+  if (!sp.split) return G;
+  const long long left = sp.left;
+  const int n = int(((tiles - left) * G + left * ((G + sp.split - 1) / sp.split)) / tiles);
+  return n < 1 ? 1 : n;
+}
+
+bool cluster_serves(int M, long long row_tiles, int K, int bits, int group_size, int chain_limit) {
   return M < kClusterMaxM && (M <= kClusterAnyM || row_tiles * ((M + 127) / 128) <= kClusterMaxTiles) && group_size >= 64 &&
-         cluster_gemm_serves(M, int(row_tiles), K, bits, group_size);
+         cluster_gemm_serves(M, int(row_tiles), K, bits, group_size, chain_limit);
 }
 
 // Host side of the persistent kernel: `nseg` projections that share x (one code stream each,
@@ -1073,16 +1090,28 @@ int persistent_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b
   PersistParams pp = {};
   pp.wait_cycles = gemm_wait_cycles();
   const bool pdl = (flags & B200LUT_FLAG_PDL) != 0, cta_pairs = (flags & B200LUT_FLAG_CTA_PAIRS) != 0;
+  int sms = 148;
   {
-    // Up to about four 128-token tiles per SM the cluster kernel is ahead (24576 x 4096: 24.7 against
-    // 37.1 us at 64 tokens, 65.7 against 86.9 at 384, even at 512; 4096 x 4096: 8.7 / 15.4 at 64, 15.1
-    // / 27.3 at 256, 27.1 / 33.4 at 768); beyond, both are held by the power cap.
+    int dev = 0;
+    B200LUT_CUDA_OK(cudaGetDevice(&dev));
+    B200LUT_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  }
+  {
+    // Up to about four 128-token tiles per SM the cluster kernel is ahead (24576 x 4096: 22.8 against
+    // 37.1 us at 64 tokens, 67.7 against 86.9 at 384, even at 512; 4096 x 4096: 9.1 / 15.4 at 64, 15.7
+    // / 27.3 at 256, 29.0 / 33.4 at 768); beyond, both are held by the power cap.
     long long row_tiles = 0;
     for (int i = 0; i < nseg; ++i) row_tiles += segs[i].N / kTileRows;
-    if (kg_rows == 0 && !(flags & B200LUT_FLAG_CTA_PAIRS) && cluster_serves(M, row_tiles, K, segs[0].bits, segs[0].group_size)) {
+    // the two launches of a two-stream projection are never cut there (their scratch holds the first one's sums)
+    const int chain = acc_out || acc_in ? K / kChunkK : persistent_chain(M, row_tiles, K / kChunkK, sms);
+    if (kg_rows == 0 && !(flags & B200LUT_FLAG_CTA_PAIRS) &&
+        cluster_serves(M, row_tiles, K, segs[0].bits, segs[0].group_size, chain)) {
       bool served = false;
+      // a workspace that the split schedule could not use means whole tiles
+      const bool refused = workspace && (!aligned16(workspace) ||
+                                         workspace_bytes < plan_split(persistent_tiles(M, row_tiles), K / kChunkK, sms).bytes);
       const int rc = cluster_gemm(x, ldx, M, K, dtype, segs, nseg, pdl, stream, acc_out, acc_in, ld_acc, pp.wait_cycles,
-                                  (flags & B200LUT_FLAG_WHOLE_TILES) != 0, false, &served);
+                                  refused || (flags & B200LUT_FLAG_WHOLE_TILES), false, chain, &served);
       if (rc != B200LUT_OK || served) return rc;
     }
   }
@@ -1125,12 +1154,6 @@ int persistent_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b
   const b200lut_segment& s = segs[0];
   pp.M = M; pp.K = K; pp.G = K / kChunkK;
   pp.gs = s.group_size;
-  int sms = 148;
-  {
-    int dev = 0;
-    B200LUT_CUDA_OK(cudaGetDevice(&dev));
-    B200LUT_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  }
   // CTA pairs (cta_group::2), on request (B200LUT_FLAG_CTA_PAIRS): the plain lookup mode only.
   // Measured 1.47x SLOWER than one CTA per tile at every prefill shape (bit-identical results),
   // so the library never picks it by itself.
@@ -1222,7 +1245,10 @@ extern "C" size_t b200lut_gemm_workspace_bytes(int M, int N, int K) {
 }
 
 extern "C" size_t b200lut_gemm_launch_workspace_bytes(int M, int N, int K, int bits, int group_size) {
-  if (M >= 1 && N >= kTileRows && cluster_serves(M, N / kTileRows, K, bits, group_size)) return 0;
+  if (M < 1 || N < kTileRows || K < 2 * kChunkK) return 0;
+  int sms = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (cluster_serves(M, N / kTileRows, K, bits, group_size, persistent_chain(M, N / kTileRows, K / kChunkK, sms))) return 0;
   return b200lut_gemm_workspace_bytes(M, N, K);
 }
 

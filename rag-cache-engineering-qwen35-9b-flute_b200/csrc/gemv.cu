@@ -830,20 +830,23 @@ bool rows_kernel_faster(const RowsGeom& g, int M) {
 // Launches that the tensor-core kernel for batches (gemm_cluster.cu) takes over, of those it serves: one
 // code stream and no residual (that factor stays fp32 here, and would be rounded to 16 bits there). Its
 // time does not depend on the rows up to 16; us here / there:
-//  * from nine rows on it is ahead everywhere (at 9 rows 4096 x 4096 9.5 / 6.8, 12288 x 4096 16.7 / 11.1,
-//    3-bit 17.2 / 11.8, 4096 x 12288 15.5 / 13.3, 1024 x 1024 6.9 / 3.9, 248320 x 4096 219 / 125; eight
-//    captured decoder layers 605 / 442);
-//  * from three rows on a launch of many row tiles per SM gains (3 rows: 128000 x 4096 75.5 / 65.5,
-//    248320 x 4096 141 / 125); at two it does not (118 / 124).
-// A step of five to eight rows would gain as well (layers 496 / 442 at five, 519 / 441 at eight), but there
-// a projection's plain launch has the bits of its launch with an exchange, with the transform inside or
-// in a persistent plan, which all run the row-range kernel.
-constexpr int kTensorCoreMinM = 9, kTensorCoreMinMHead = 3;
-constexpr int kTensorCoreHeadTiles = 1000;
+//  * from nine rows on it is ahead (at 9 rows 4096 x 4096 9.3 / 8.5, 12288 x 4096 16.0 / 11.5, 3-bit
+//    16.5 / 12.3, 4096 x 12288 15.2 / 14.3, 1024 x 1024 6.9 / 4.7, 512 x 4096 6.0 / 6.1, 248320 x 4096 220 / 126),
+//  * but for launches of 8 to 15 row tiles and more than 32 k-blocks, which the tile kernel cuts eight ways
+//    in one wave (1024 x 4096 6.7 / 7.6, 1920 x 4096 7.5 / 8.7; 2048 x 4096, two waves there, 12.9 / 7.6;
+//    1920 x 2048 6.5 / 5.7).
+// Five to eight rows would gain as well, and a large head from three (248320 x 4096 141 / 125), but up to
+// eight rows a projection's plain launch has the bits of its launch with an exchange, with the transform
+// inside or in a persistent plan, which all run the row-range kernel.
+// Each of its accumulators sums at most the k-blocks that one warp of the tile kernel, which would serve the
+// launch otherwise, sums in its own (the tensor core truncates where it accumulates, so a longer chain is a
+// larger error): with one chain per CTA 1.7e-2 of the fp16 results of 12288 x 4096 were not the rounding of
+// the 64-bit sum, 2.8e-3 in the tile kernel.
+constexpr int kTensorCoreMinM = 9;
 
 bool tensor_core_decode(const GemvParams& p, int flags) {
-  const int min_m = p.seg[0].bits == 4 && p.tiles_total >= kTensorCoreHeadTiles ? kTensorCoreMinMHead : kTensorCoreMinM;
-  if (p.M < min_m || p.nseg > 4 || p.G < 2) return false;
+  if (p.M < kTensorCoreMinM || p.nseg > 4 || p.G < 2) return false;
+  if (p.tiles_total >= 8 && p.tiles_total < 16 && p.G > 32) return false;
   if ((flags & (B200LUT_FLAG_TILE_KERNEL | B200LUT_FLAG_ROWS_KERNEL)) || !rows_kernel_wanted(0)) return false;
   if (p.epilogue == B200LUT_EPI_SILU_MUL && p.nseg != 2) return false;
   for (int i = 0; i < p.nseg; ++i) {
@@ -1165,8 +1168,9 @@ extern "C" int b200lut_gemv_input(const void* x, int64_t ldx, int M, int K, int 
   cudaStream_t st = cudaStream_t(stream);
   if (split <= 0 && !transformed && !p.ex.push && !p.ex.wait && tensor_core_decode(p, flags)) {
     bool served = false;
+    const int blocks = pick_split(tiles, p.G, sm_count_cached(), kWarpsM16), per_block = (p.G + blocks - 1) / blocks;
     const int rc = cluster_gemm(x, ldx, M, K, dtype, segs, nseg, pdl, stream, nullptr, nullptr, 0, gemm_wait_cycles(),
-                                false, silu, &served);
+                                false, silu, (per_block + kWarpsM16 - 1) / kWarpsM16, &served);
     if (rc || served) return rc;
   }
   // Library policy (split == 0): the row-range kernel when it serves the shapes. An explicit

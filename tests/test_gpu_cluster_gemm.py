@@ -79,7 +79,7 @@ def test_merged_projections_with_and_without_a_residual():
     (128, 832, 256, 2, torch.float16, 12, False),
     (256, 1088, 512, 1, torch.bfloat16, 16, True),
     (19200, 192, 128, 4, torch.bfloat16, 10, False),                   # 150 row tiles
-    (128 * 1000, 128, 128, 4, torch.bfloat16, 3, False),               # the fewest rows of many row tiles
+    (128 * 1000, 128, 128, 4, torch.bfloat16, 3, False),               # few rows of many row tiles (not this kernel)
 ))
 def test_batched_decode(N, K, gs, bits, dtype, M, bias):
     case = Case(N, K, gs, bits, dtype, seed=N + K + M, bias=bias)
@@ -156,3 +156,46 @@ def test_cut_gated_tiles_one_after_the_other(N, M):
         out.fill_(float("nan"))
         L.gemv_multi(x, segs, 2, epilogue=L.EPI_SILU_MUL)
         assert rel_err(out, (torch.nn.functional.silu(g) * u).float()) <= 2.0 ** -8
+
+
+def _missed(mod, x, **kw):
+    """Share of fp16 outputs that are not the rounding of the 64-bit sums (one launch of `mod` over x)."""
+    mod._ensure_packed()
+    out = torch.empty(x.shape[0], mod.N, dtype=x.dtype, device="cuda")
+    seg = L.make_segments([mod._segment_desc(out)])
+    L.gemv_multi(x, seg, 1, **kw) if x.shape[0] <= 16 else L.gemm(x, seg, **kw)
+    want = x.double() @ mod._quantized_weight().double().t()
+    return (out != want.to(x.dtype)).double().mean().item(), out
+
+
+@pytest.mark.parametrize("N,K,bits,gs,M", (
+    (12288, 4096, 3, 64, 16),        # one CTA per tile: eight chains
+    (4096, 4096, 4, 128, 9),         # cut tiles
+    (4096, 12288, 4, 128, 12),
+    (1024, 1024, 2, 128, 16),        # single k-blocks
+))
+def test_batched_decode_sums_no_less_exactly_than_the_tile_kernel(N, K, bits, gs, M):
+    # both truncate at every accumulation of the tensor core and round where chains are added; with chains
+    # of equal length the shares are those of two samples of one population, four deviations apart at most
+    # (one chain per CTA: 5 to 10 times the tile kernel's share)
+    mod = _synthetic(N, K, bits, gs)
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).half().cuda()
+    here, tile = _missed(mod, x)[0], _missed(mod, x, flags=L.FLAG_TILE_KERNEL)[0]
+    assert here <= tile + 4 * (2 * max(tile, 1 / (M * N)) / (M * N)) ** 0.5
+
+
+@pytest.mark.parametrize("N,K,bits,gs,M", ((4096, 4096, 4, 128, 64), (4096, 4096, 4, 128, 128), (1024, 1024, 2, 128, 700)))
+def test_short_prompts_sum_in_chains_of_a_quarter_of_k(N, K, bits, gs, M):
+    # the whole-tile kernel's split schedule cuts these tiles into four parts or more: a quarter of the
+    # truncations behind one another; the fp32 additions of the parts round (2^-24 of the value each, 2^-13
+    # of fp16's spacing, a few of them on partial sums up to a few times the result: 1.5e-3 at most)
+    mod = _synthetic(N, K, bits, gs)
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).half().cuda()
+    assert _missed(mod, x)[0] <= _missed(mod, x, split=False)[0] / 4 + 1.5e-3
+
+
+@pytest.mark.parametrize("M", (3, 8))
+def test_a_head_of_few_rows_has_the_bits_of_the_row_range_kernel(M):
+    mod = _synthetic(128 * 1000, 128, 4, 128)
+    x = torch.randn(M, 128, generator=torch.Generator().manual_seed(M)).half().cuda()
+    assert torch.equal(_missed(mod, x)[1], _missed(mod, x, flags=L.FLAG_ROWS_KERNEL)[1])
