@@ -649,6 +649,23 @@ def _merged_decode(owner: nn.Module, mods, x: torch.Tensor, epilogue: int = None
     return out
 
 
+_LINEAR_FORWARD, _MODULE_CALL = PalettizedLinear.forward, nn.Module.__call__
+
+
+def _call_is_forward(m) -> bool:
+    """Calling `m` runs PalettizedLinear.forward and nothing else: no subclass, no replaced forward, no hook
+    of its own or of all modules, no compiled call."""
+    d = m.__dict__
+    if type(m) is not PalettizedLinear or PalettizedLinear.forward is not _LINEAR_FORWARD or "forward" in d:
+        return False
+    if nn.Module.__call__ is not _MODULE_CALL or d.get("_compiled_call_impl") is not None:
+        return False
+    g = nn.modules.module
+    return not (d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"]
+                or g._global_forward_hooks or g._global_forward_pre_hooks
+                or g._global_backward_hooks or g._global_backward_pre_hooks)
+
+
 def _bind_all(mods) -> None:
     for m in mods:
         if isinstance(m, PalettizedLinear):
@@ -716,7 +733,10 @@ class FusedPalettizedMLP(nn.Module):
         return out
 
     def forward(self, x):
-        out = _lib.host.mlp(self.__dict__, x, _LAUNCH_FLAGS["pdl"]) if self._is_silu() else None
+        # the native route computes all three projections, so it is for a down projection whose call
+        # is its forward and nothing else
+        native = self._is_silu() and _call_is_forward(self.down_proj)
+        out = _lib.host.mlp(self.__dict__, x, _LAUNCH_FLAGS["pdl"]) if native else None
         if out is None:
             out = self._forward_route(x)
             _bind_all((self.gate_proj, self.up_proj, self.down_proj))

@@ -88,3 +88,37 @@ def test_scratch_of_a_captured_graph_is_its_own():
         assert torch.equal(mod(x), want)
         torch.cuda.synchronize()
         assert torch.equal(o, want)
+
+
+class _Doubled(pkg.PalettizedLinear):
+    def forward(self, x):
+        return 2 * super().forward(x)
+
+
+def _double_forward(m):
+    plain = m.forward
+    m.forward = lambda x: 2 * plain(x)
+
+
+@pytest.mark.parametrize("attach", (
+    lambda m: m.register_forward_hook(lambda mod, args, out: 2 * out),
+    lambda m: m.register_forward_pre_hook(lambda mod, args: (2 * args[0],)),
+    lambda m: torch.nn.modules.module.register_module_forward_hook(lambda mod, args, out: 2 * out if mod is m else None),
+    _double_forward,
+    lambda m: setattr(m, "__class__", _Doubled),
+), ids=("hook", "pre_hook", "global_hook", "instance_forward", "subclass"))
+@pytest.mark.parametrize("M", (1, 16, 40))
+def test_what_is_attached_to_the_down_projection_runs_in_every_call(M, attach):
+    K, inner = 256, 384
+    mk = lambda n, k, s: Case(n, k, 128, 4, torch.bfloat16, seed=s).module()     # noqa: E731
+    mlp = pkg.FusedPalettizedMLP(mk(inner, K, 4), mk(inner, K, 5), mk(K, inner, 6), torch.nn.SiLU())
+    x = torch.randn(M, K, device="cuda").bfloat16()
+    want = 2 * mlp(x)                                   # exact: a power of two
+    mlp(x)
+    handle = attach(mlp.down_proj)
+    try:
+        for _ in range(3):
+            assert torch.equal(mlp(x), want)
+    finally:
+        if hasattr(handle, "remove"):
+            handle.remove()
