@@ -11,7 +11,7 @@ using namespace b200host;
 
 namespace b200host {
 
-// ---- Layer and Stack objects ----------------------------------------------------------------------
+// ---- Layer objects ----------------------------------------------------------------------
 static void layer_clear(Layer* l) {
   for (at::Tensor* t : {l->packed, l->lut, l->packed2, l->lut2, l->bias, l->resA, l->resB, l->signs, l->awq}) delete t;
   if (l->watches) {
@@ -27,20 +27,13 @@ static void layer_dealloc(PyObject* o) {
   layer_clear(reinterpret_cast<Layer*>(o));
   PyObject_Free(o);
 }
-static void stack_dealloc(PyObject* o) {
-  Stack* s = reinterpret_cast<Stack*>(o);
-  delete s->resB;
-  Py_XDECREF(s->keep);
-  PyObject_Free(o);
-}
-// A copied or pickled module builds its own description: these objects travel as None.
+// A copied or pickled module builds its own description: this object travels as None.
 static PyObject* reduce_none(PyObject*, PyObject*) {
   return Py_BuildValue("(O())", reinterpret_cast<PyObject*>(Py_TYPE(Py_None)));
 }
 static PyMethodDef reduce_methods[] = {{"__reduce__", reduce_none, METH_NOARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
 
 PyTypeObject LayerType = {PyVarObject_HEAD_INIT(nullptr, 0)};
-PyTypeObject StackType = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
 static int ready_type(PyTypeObject* t, const char* name, size_t size, destructor d) {
   t->tp_name = name;
@@ -191,7 +184,7 @@ static PyObject* qkv(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     Rows r;
     Ctx c;
-    if (!rows_of(x, *ls[0], &r) || !mergeable(ls, 3, r.M) || !context(ls[0]->device, a[2] == Py_True, &c)) Py_RETURN_NONE;
+    if (!rows_of(x, *ls[0], &r) || !mergeable(a[0], ls, 3, r.M) || !context(ls[0]->device, a[2] == Py_True, &c)) Py_RETURN_NONE;
     at::Tensor out = output_like(x, total, *ls[0]);
     char* p = static_cast<char*>(out.mutable_data_ptr());
     void* outs[3];
@@ -220,7 +213,7 @@ static PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Rows r;
     Ctx c;
     if (!rows_of(x, *ls[0], &r) || ls[1]->N != I || down.K != I || down.dtype != ls[0]->dtype ||
-        down.device != ls[0]->device || !mergeable(ls, 2, r.M) || linear_kind(down, r.M) == Kind::kNotServed ||
+        down.device != ls[0]->device || !mergeable(a[0], ls, 2, r.M) || linear_kind(down, r.M) == Kind::kNotServed ||
         !context(down.device, a[2] == Py_True, &c))
       Py_RETURN_NONE;
     at::Tensor g = empty({r.M, I}, down.scalar, down.device), u;
@@ -369,8 +362,6 @@ static PyModuleDef module = {PyModuleDef_HEAD_INIT, "_b200lut_host", nullptr, -1
 }  // namespace b200host
 
 PyMODINIT_FUNC PyInit__b200lut_host(void) {
-  if (ready_type(&LayerType, "_b200lut_host.Layer", sizeof(Layer), layer_dealloc) < 0 ||
-      ready_type(&StackType, "_b200lut_host.Stack", sizeof(Stack), stack_dealloc) < 0)
-    return nullptr;
+  if (ready_type(&LayerType, "_b200lut_host.Layer", sizeof(Layer), layer_dealloc) < 0) return nullptr;
   return PyModule_Create(&module);
 }

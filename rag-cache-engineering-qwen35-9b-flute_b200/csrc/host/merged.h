@@ -7,49 +7,34 @@ namespace b200host {
 
 constexpr int kMaxMerged = 4;
 
-// The residual's first factors of the merged projections, stacked along r so that one projection
-// launch serves them all; kept in the owning module's __dict__ and rebuilt when a factor changes.
-struct Stack {
-  PyObject_HEAD
-  int n, cols;                     // layers, columns of t
-  Layer* layers[kMaxMerged];       // borrowed for identity; `keep` owns them
-  PyObject* keep;
-  int offset[kMaxMerged];          // first row of each layer's factor
-  at::Tensor* resB;
-};
-extern PyTypeObject StackType;
+// The residual's first factors of the merged projections, stacked along r so that one projection launch
+// serves them all: the record that the Python route keeps in the owning module's __dict__ as "_resB_stack",
+// (stack, factors, (address, version) of each factor). Null when there is none for the factors as they are
+// now; the Python route then builds it, outside of any stream capture.
+inline PyObject* name_stack() { static PyObject* s = PyUnicode_InternFromString("_resB_stack"); return s; }
 
-inline PyObject* name_stack() { static PyObject* s = PyUnicode_InternFromString("_native_stack"); return s; }
-
-inline Stack* stack_of(PyObject* owner_dict, Layer* const* ls, int n) {
+inline const at::Tensor* residual_stack(PyObject* owner_dict, Layer* const* ls, int n) {
   PyObject* o = PyDict_GetItemWithError(owner_dict, name_stack());
-  if (o && Py_TYPE(o) == &StackType) {
-    Stack* st = reinterpret_cast<Stack*>(o);
-    bool same = st->n == n && st->resB;
-    for (int i = 0; same && i < n; ++i) same = st->layers[i] == ls[i];
-    if (same) return st;
-  }
-  Stack* st = PyObject_New(Stack, &StackType);
-  if (!st) throw LaunchError(0, "out of memory");
-  st->n = n;
-  st->resB = nullptr;
-  st->keep = PyList_New(0);
-  std::vector<at::Tensor> parts;
-  int off = 0;
+  if (!o || !PyTuple_Check(o) || PyTuple_GET_SIZE(o) != 3) return nullptr;
+  PyObject *stack = PyTuple_GET_ITEM(o, 0), *factors = PyTuple_GET_ITEM(o, 1), *marks = PyTuple_GET_ITEM(o, 2);
+  if (!THPVariable_Check(stack) || !PyTuple_Check(factors) || !PyTuple_Check(marks) ||
+      PyTuple_GET_SIZE(marks) != 2 * PyTuple_GET_SIZE(factors))
+    return nullptr;
+  Py_ssize_t at_factor = 0;
   for (int i = 0; i < n; ++i) {
-    st->layers[i] = ls[i];
-    PyList_Append(st->keep, reinterpret_cast<PyObject*>(ls[i]));
-    st->offset[i] = off;
-    if (ls[i]->res) {
-      parts.push_back(*ls[i]->resB);
-      off += int(ls[i]->resB->size(0));
-    }
+    if (!ls[i]->res) continue;
+    const at::Tensor& b = *ls[i]->resB;
+    if (at_factor >= PyTuple_GET_SIZE(factors)) return nullptr;
+    PyObject* f = PyTuple_GET_ITEM(factors, at_factor);
+    if (!THPVariable_Check(f) || !THPVariable_Unpack(f).is_same(b)) return nullptr;
+    const unsigned long long address = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(marks, 2 * at_factor));
+    const long long version = PyLong_AsLongLong(PyTuple_GET_ITEM(marks, 2 * at_factor + 1));
+    if (PyErr_Occurred()) { PyErr_Clear(); return nullptr; }
+    if (address != reinterpret_cast<uintptr_t>(b.const_data_ptr()) || version != (b.is_inference() ? -1 : b._version()))
+      return nullptr;
+    ++at_factor;
   }
-  st->cols = off;
-  st->resB = new at::Tensor(at::cat(parts, 0).contiguous());
-  PyDict_SetItem(owner_dict, name_stack(), reinterpret_cast<PyObject*>(st));
-  Py_DECREF(st);                   // the dict holds it
-  return st;
+  return at_factor == PyTuple_GET_SIZE(factors) ? &THPVariable_Unpack(stack) : nullptr;
 }
 
 inline bool same_fold(const Layer& a, const Layer& b) {
@@ -57,17 +42,19 @@ inline bool same_fold(const Layer& a, const Layer& b) {
   return a.rotation && b.rotation && PyObject_RichCompareBool(a.rotation, b.rotation, Py_EQ) == 1;
 }
 
-// One dtype, K and fold; every residual of a kind the launch carries.
-inline bool mergeable(Layer* const* ls, int n, int M) {
+// One dtype, K and fold; every residual of a kind the launch carries (at decode with its stack at hand).
+inline bool mergeable(PyObject* owner_dict, Layer* const* ls, int n, int M) {
   if (env_on("FLUTE_NO_MERGE")) return false;
   const Layer& a = *ls[0];
+  bool any_res = false;
   for (int i = 0; i < n; ++i) {
     const Layer& l = *ls[i];
+    any_res = any_res || l.res;
     if (l.kgrouped || l.K != a.K || l.dtype != a.dtype || l.device != a.device || !same_fold(a, l)) return false;
     if (l.res && !residual_served(l, M)) return false;
     if (M > kGemvMaxM && (l.K < 128 || l.two || l.bits != a.bits || l.group != a.group || l.group < 64)) return false;
   }
-  return true;
+  return !any_res || M > kGemvMaxM || residual_stack(owner_dict, ls, n) != nullptr;
 }
 
 // The merged launch into outs[i] (row stride ld): M <= 16 the decode kernels, with EPI_SILU_MUL only
@@ -93,13 +80,17 @@ inline void merged_into(PyObject* owner_dict, Layer* const* ls, int n, Rows r, v
   }
   if (r.M <= kGemvMaxM) {
     if (any_res) {
-      Stack* st = stack_of(owner_dict, ls, n);
-      t = empty({r.M, st->cols}, at::kFloat, c.device);
+      const at::Tensor& stack = *residual_stack(owner_dict, ls, n);
+      const int cols = int(stack.size(0));
+      t = empty({r.M, cols}, at::kFloat, c.device);
       float* tp = static_cast<float*>(t.mutable_data_ptr());
-      check(b200lut_residual_project(r.ptr, r.ld, r.M, a.K, a.dtype, st->resB->const_data_ptr(), st->cols, tp, st->cols,
-                                     c.flags, c.stream));
-      for (int i = 0; i < n; ++i)
-        if (ls[i]->res) add_residual(&segs[i], *ls[i], tp + st->offset[i], st->cols);
+      check(b200lut_residual_project(r.ptr, r.ld, r.M, a.K, a.dtype, stack.const_data_ptr(), cols, tp, cols, c.flags,
+                                     c.stream));
+      for (int i = 0; i < n; ++i) {
+        if (!ls[i]->res) continue;
+        add_residual(&segs[i], *ls[i], tp, cols);
+        tp += ls[i]->resB->size(0);
+      }
     }
     if (fused) {
       b200lut_input in = {};

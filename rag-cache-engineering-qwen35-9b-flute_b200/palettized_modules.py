@@ -597,12 +597,19 @@ def _stacked_residual(owner: nn.Module, mods, x2: torch.Tensor):
     with_res = [m for m in mods if m.has_residual()]
     if not with_res:
         return {}
-    key = tuple(m.resB.data_ptr() for m in with_res)
+    # (stack, factors, their addresses and versions): rebuilt when a factor is another tensor, has other
+    # storage or was written to. The native host layer reads this record too (csrc/host/merged.h).
+    factors = tuple(m.resB for m in with_res)
+    marks = tuple(v for f in factors for v in (f.data_ptr(), -1 if f.is_inference() else f._version))
     cache = owner.__dict__.get("_resB_stack")
-    if cache is None or cache[0] != key:
-        cache = (key, torch.cat([m.resB for m in with_res], dim=0).contiguous())
-        owner.__dict__["_resB_stack"] = cache
-    t = _lib.residual_project(x2, cache[1], flags=_flags())
+    if cache is None or len(cache[1]) != len(factors) or any(a is not b for a, b in zip(cache[1], factors)) \
+            or cache[2] != marks:
+        cache = (torch.cat(factors, dim=0).contiguous(), factors, marks)
+        # under stream capture the concatenation is only recorded: this graph runs it in every replay, and
+        # what is kept for other calls is filled by an eager one
+        if not torch.cuda.is_current_stream_capturing():
+            owner.__dict__["_resB_stack"] = cache
+    t = _lib.residual_project(x2, cache[0], flags=_flags())
     out, off = {}, 0
     for m in with_res:
         r = m.resB.shape[0]

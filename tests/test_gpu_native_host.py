@@ -122,3 +122,45 @@ def test_what_is_attached_to_the_down_projection_runs_in_every_call(M, attach):
     finally:
         if hasattr(handle, "remove"):
             handle.remove()
+
+
+def _merged_with_residuals(K=256, inner=384):
+    mk = lambda n, k, s, r: Case(n, k, 128, 4, torch.float16, seed=s, residual=r).module()     # noqa: E731
+    return (pkg.SplitQKV(mk(256, K, 1, 16), mk(128, K, 2, 0), mk(128, K, 3, 8)),
+            pkg.FusedPalettizedMLP(mk(inner, K, 4, 8), mk(inner, K, 5, 24), mk(K, inner, 6, 16), torch.nn.SiLU()))
+
+
+@pytest.mark.parametrize("which", (0, 1), ids=("qkv", "mlp"))
+@pytest.mark.parametrize("warm_up_rows", (4, 40))          # 40: the decode step's first call is the captured one
+def test_residuals_of_graphs_and_eager_calls_do_not_depend_on_a_replay(which, warm_up_rows):
+    mod = _merged_with_residuals()[which]
+    xs = [torch.randn(m, 256, device="cuda").half() for m in (2, 3)]
+    wants = [_merged_with_residuals()[which](x) for x in xs]
+    mod(torch.randn(warm_up_rows, 256, device="cuda").half())
+    torch.cuda.synchronize()
+    graphs, outs = [], []
+    for x in xs:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            outs.append(mod(x))
+        graphs.append(g)
+    for _ in range(2):                                      # eager calls before any replay
+        assert all(torch.equal(mod(x), w) for x, w in zip(xs, wants))
+    for i in (1, 0, 1):                                     # the second graph first
+        graphs[i].replay()
+        torch.cuda.synchronize()
+        assert torch.equal(outs[i], wants[i])
+    assert all(torch.equal(mod(x), w) for x, w in zip(xs, wants))
+
+
+@pytest.mark.parametrize("which", (0, 1), ids=("qkv", "mlp"))
+def test_a_residual_factor_written_in_place_is_followed(which):
+    mod = _merged_with_residuals()[which]
+    x = torch.randn(3, 256, device="cuda").half()
+    mod(x), mod(x)
+    first = mod.q_proj if which == 0 else mod.gate_proj
+    other = _merged_with_residuals()[which]
+    for m in (first, other.q_proj if which == 0 else other.gate_proj):
+        m.resB.mul_(-3)
+    want = other(x)                                         # stacked after the change
+    assert torch.equal(mod(x), want) and torch.equal(mod._forward_route(x), want) and torch.equal(mod(x), want)
