@@ -27,7 +27,9 @@
 //    above). Where they do not fit into half of the columns, a tile takes both halves and the next tile's
 //    MMAs start when they have been read.
 // Weights are the A operand in tensor memory, tokens (up to 128 per tile) the B operand in shared
-// memory, as in gemm_tc.cu. All waits are bounded.
+// memory, as in gemm_tc.cu. All waits are bounded, and a wait that depends on the activations starts after
+// the previous kernel has ended (an exchange may keep that one waiting for a peer for up to a second): the
+// lookup warps' second stage, the code producer's second round of its ring, the MMA issuer.
 //
 // The gated form (kModeGated, up to 16 tokens): a cluster takes a row tile of gate and then the same row
 // tile of up, and an epilogue thread, which finishes the same eight outputs of both, holds the finished
@@ -295,6 +297,7 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
         if (lane == 0) tc::mbar_arrive(bar_cempty + 8 * slot);
         slot += kCGroups;
         if (slot >= nc) { slot -= nc; cphase ^= 1u; }
+        if (st == grp + kCGroups) asm volatile("griddepcontrol.wait;" ::: "memory");   // the first wait for an MMA
         tc::mbar_wait(bar_done + 8 * grp, dphase, abort_flag, &g_cluster_status, tc::kStatusWaitEmpty, lim);
         dphase ^= 1u;
         tc::fence_after_sync();
@@ -369,7 +372,11 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
             tc::mbar_expect_tx(bar, bytes);
             bulk_load(codes + uint32_t(slot) * slot_bytes, src, bytes, bar, policy);
           }
-          if (++slot == nc) { slot = 0; phase ^= 1u; }
+          if (++slot == nc) {
+            if (phase) asm volatile("griddepcontrol.wait;" ::: "memory");   // from here on slots come back from the lookups
+            slot = 0;
+            phase ^= 1u;
+          }
         }
       }
     }
@@ -403,6 +410,7 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
     __syncwarp();
   } else if (warp == kCMmaWarp) {
     // ---- MMA issuer: a short loop, eight MMAs and one commit per stage ------------------------------------
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (tc::elect_one()) {
       constexpr uint32_t kFmt = DType<T>::id == B200LUT_BF16 ? 1u : 0u;
       const uint32_t idesc = tc::instr_desc(kFmt, 128, uint32_t(p.NT));

@@ -199,3 +199,28 @@ def test_a_head_of_few_rows_has_the_bits_of_the_row_range_kernel(M):
     mod = _synthetic(128 * 1000, 128, 4, 128)
     x = torch.randn(M, 128, generator=torch.Generator().manual_seed(M)).half().cuda()
     assert torch.equal(_missed(mod, x)[1], _missed(mod, x, flags=L.FLAG_ROWS_KERNEL)[1])
+
+
+def test_a_launch_behind_a_long_exchange_wait_does_not_give_up():
+    # the exchange waits 60 ms for rows that nobody pushes (it reports that, and ends); the launch behind it
+    # starts early on the SMs that are free, and its own waits are bounded by 10 ms
+    from importlib import import_module
+    exchange = import_module(pkg.__name__ + ".exchange")
+    M, dt = 16, torch.bfloat16
+    arena = exchange.PeerArena.emulated(1 << 16, 2, "cuda")[0]
+    cons = _synthetic(128, 256, 4, 128, dt)
+    mod = _synthetic(4096, 1024, 4, 128, dt)
+    for m in (cons, mod):
+        m._ensure_packed()
+    x = torch.randn(M, 1024, generator=torch.Generator().manual_seed(1)).to(dt).cuda()
+    y, out, want = (torch.zeros(M, n, dtype=dt, device="cuda") for n in (128, 4096, 4096))
+    L.gemv_multi(x, L.make_segments([mod._segment_desc(want)]), 1)
+    torch.cuda.synchronize()
+    blocks = L.gemv_launch_blocks(M, 256, L.make_segments([cons._segment_desc(None)]), 1)
+    chan = exchange.Channel(arena, M, 256, dt, blocks)
+    chan.wait.wait_ms = 60
+    L.gemv_exchange(chan.act, L.make_segments([cons._segment_desc(y)]), 1, chan.wait)
+    L.gemv_multi(x, L.make_segments([mod._segment_desc(out)]), 1, flags=L.FLAG_PDL)
+    torch.cuda.synchronize()
+    assert L.lib().b200lut_device_status() in (0x7000, 0x7001)        # the exchange's, not a pipeline wait's
+    assert torch.equal(out, want)
