@@ -611,6 +611,15 @@ gemm_tc_persistent_kernel_clusters(const __grid_constant__ CUtensorMap xmap, con
       }
     }
   }
+  // A wait has given up: copies into this CTA's memory, sums sent to other CTAs and MMAs may be under way with
+  // nobody to wait for them. They take microseconds; every thread that ends its role after the flag was set
+  // stays for 100000 cycles (50 us), so the CTA leaves, and frees its tensor memory, behind all of them.
+  __syncwarp();
+  if (__any_sync(0xffffffffu, *abort_flag != 0)) {
+    const long long t0 = clock64();
+    while (clock64() - t0 < 100000) { }
+    __syncwarp();
+  }
   tc::fence_before_sync();
   // A CTA must not leave while another's sums are on their way to it. It has waited for all of them —
   // unless a wait gave up, so the CTAs meet; by now every arrival of the others is near.
