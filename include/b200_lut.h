@@ -52,8 +52,9 @@ enum {
                                     covers 256 weight rows, each CTA fetches half of the activation
                                     tile; no multicast load). Same results bit for bit, measured
                                     slower than one CTA per tile, so it is never the default */
-  B200LUT_FLAG_WHOLE_TILES = 16  /* prefill GEMM: every output is one sum over all of K (no cut of K over
-                                    the blocks of a cluster) */
+  B200LUT_FLAG_WHOLE_TILES = 16  /* prefill GEMMs: every output (of two streams, each stream's part) is one sum
+                                    over all of K: no cut of K over blocks, whatever the workspace, and one
+                                    accumulator */
 };
 
 /* Epilogue selector of b200lut_gemv_multi / b200lut_gemm. */

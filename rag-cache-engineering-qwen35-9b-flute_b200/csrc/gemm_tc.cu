@@ -1179,7 +1179,7 @@ int persistent_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b
   if (pair) sp.bytes = sp.split ? kTicketBytes + 2 * (sp.bytes - kTicketBytes) : 0;   // a slot per CTA
   if (pair && sp.left > int(kTicketBytes / 16)) sp.split = 0;
   if (sp.split && workspace && workspace_bytes >= sp.bytes && aligned16(workspace) &&
-      !acc_out && !acc_in) {
+      !(flags & B200LUT_FLAG_WHOLE_TILES) && !acc_out && !acc_in) {
     pp.split = sp.split; pp.full = sp.full; pp.left = sp.left;
     pp.tickets = static_cast<int*>(workspace);
     pp.ws = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + kTicketBytes);
@@ -1349,11 +1349,9 @@ extern "C" int b200lut_gemm_two_stream(const void* x, int64_t ldx, int M, int K,
   first.res_rank = 0; first.resA = nullptr; first.res_t = nullptr;   // the second launch carries it
   second.packed = s.packed2; second.lut = s.lut2; second.bits = s.bits2;
   second.packed2 = second.lut2 = nullptr; second.bits2 = 0;
-  if (int rc = persistent_gemm(x, ldx, M, K, dtype, &first, 1, flags & B200LUT_FLAG_PDL, nullptr, 0, stream, acc,
-                               nullptr, s.N))
-    return rc;
-  return persistent_gemm(x, ldx, M, K, dtype, &second, 1, flags & B200LUT_FLAG_PDL, nullptr, 0, stream, nullptr, acc,
-                         s.N);
+  flags &= B200LUT_FLAG_PDL | B200LUT_FLAG_WHOLE_TILES;
+  if (int rc = persistent_gemm(x, ldx, M, K, dtype, &first, 1, flags, nullptr, 0, stream, acc, nullptr, s.N)) return rc;
+  return persistent_gemm(x, ldx, M, K, dtype, &second, 1, flags, nullptr, 0, stream, nullptr, acc, s.N);
 }
 
 extern "C" int b200lut_gemm_ws(const void* x, int64_t ldx, int M, int K, int dtype,

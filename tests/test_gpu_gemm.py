@@ -353,3 +353,41 @@ def test_cta_pairs_give_the_same_bits_as_single_ctas(N, K, gs, bits, dtype, M, b
     d["out"].fill_(float("nan"))
     L.gemm(x, L.make_segments([d]), flags=L.FLAG_CTA_PAIRS)     # cut tiles: other K split points
     assert rel_err(d["out"], single) <= 4e-3
+
+
+def test_the_whole_tiles_flag_keeps_every_launch_from_cutting_k():
+    stream = lambda x: L._stream(x)                                                             # noqa: E731
+    # the persistent kernel (more rows than the cluster kernel takes) with a workspace it could use
+    N, K, M = 512, 2048, 1100
+    case = Case(N, K, 128, 3, torch.float16, seed=21)
+    mod = case.module()
+    mod._ensure_packed()
+    x = case.x(M).cuda()
+    need = L.lib().b200lut_gemm_launch_workspace_bytes(M, N, K, 3, 128)
+    assert need > 0
+    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    outs = [torch.empty(M, N, dtype=torch.float16, device="cuda") for _ in range(3)]
+    for out, flags, ptr, size in zip(outs, (0, L.FLAG_WHOLE_TILES, 0), (None, ws.data_ptr(), ws.data_ptr()), (0, need, need)):
+        L.check(L.lib().b200lut_gemm_ws(x.data_ptr(), K, M, K, L.dtype_id(x.dtype), L.make_segments([mod._segment_desc(out)]),
+                                        0, flags, ptr, size, stream(x)))
+    assert torch.equal(outs[1], outs[0]) and not torch.equal(outs[2], outs[0])
+    # palettes along K
+    lut_k = (0.02 * torch.randn(K // 128, N, 16, generator=torch.Generator().manual_seed(3))).half().cuda()
+    packed = torch.randint(0, 256, (N * K // 2,), dtype=torch.uint8, device="cuda")
+    need = L.lib().b200lut_gemm_workspace_bytes(M, N, K)
+    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    for out, flags, ptr, size in zip(outs, (0, L.FLAG_WHOLE_TILES), (None, ws.data_ptr()), (0, need)):
+        L.check(L.lib().b200lut_gemm_kgrouped(x.data_ptr(), K, M, K, L.dtype_id(x.dtype), packed.data_ptr(), lut_k.data_ptr(),
+                                              None, N, 4, out.data_ptr(), N, flags, ptr, size, stream(x)))
+    assert torch.equal(outs[1], outs[0])
+    # two streams, the second one of zeros: the first one's whole sums, rounded
+    two = Case(256, 4096, 128, 4, torch.float16, seed=22, bits2=2)
+    two.kw["lut2"].zero_()
+    mod = two.module()
+    mod._ensure_packed()
+    x = two.x(64).cuda()
+    got, want = (torch.empty(64, 256, dtype=torch.float16, device="cuda") for _ in range(2))
+    L.gemm_two_stream(x, L.make_segments([mod._segment_desc(got)]), flags=L.FLAG_WHOLE_TILES)
+    one = {k: v for k, v in mod._segment_desc(want).items() if k not in ("packed2", "lut2", "bits2")}
+    L.gemm(x, L.make_segments([one]), split=False)
+    assert torch.equal(got, want)
