@@ -656,6 +656,11 @@ def _merged_decode(owner: nn.Module, mods, x: torch.Tensor, epilogue: int = None
     return out
 
 
+def _on_cuda(x) -> bool:
+    """Whether the native host layer may serve x; the library is not loaded for anything else."""
+    return torch.is_tensor(x) and x.is_cuda
+
+
 _LINEAR_FORWARD, _MODULE_CALL = PalettizedLinear.forward, nn.Module.__call__
 
 
@@ -688,7 +693,7 @@ class SplitQKV(nn.Module):
         self.q_proj, self.k_proj, self.v_proj = q_proj, k_proj, v_proj
 
     def forward(self, x):
-        out = _lib.host.qkv(self.__dict__, x, _LAUNCH_FLAGS["pdl"])
+        out = _lib.host.qkv(self.__dict__, x, _LAUNCH_FLAGS["pdl"]) if _on_cuda(x) else None
         if out is None:
             out = self._forward_route(x)
             _bind_all((self.q_proj, self.k_proj, self.v_proj))
@@ -742,7 +747,7 @@ class FusedPalettizedMLP(nn.Module):
     def forward(self, x):
         # the native route computes all three projections, so it is for a down projection whose call
         # is its forward and nothing else
-        native = self._is_silu() and _call_is_forward(self.down_proj)
+        native = _on_cuda(x) and self._is_silu() and _call_is_forward(self.down_proj)
         out = _lib.host.mlp(self.__dict__, x, _LAUNCH_FLAGS["pdl"]) if native else None
         if out is None:
             out = self._forward_route(x)
@@ -1099,7 +1104,7 @@ class KGroupedPalettizedLinear(nn.Module):
             self.__dict__["_native"] = _lib.host.bind(self.__dict__, spec)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        out = _lib.host.kgrouped(self.__dict__, x, _LAUNCH_FLAGS["pdl"])
+        out = _lib.host.kgrouped(self.__dict__, x, _LAUNCH_FLAGS["pdl"]) if _on_cuda(x) else None
         if out is None:
             out = self._forward_route(x)
             self._bind()

@@ -256,3 +256,21 @@ def test_missing_library_is_loud(monkeypatch):
     monkeypatch.setattr(pkg._lib, "LIB_PATH", "/nonexistent/libb200lut.so")
     with pytest.raises(RuntimeError, match="missing"):
         pkg._lib.lib()
+
+
+def test_modules_on_the_cpu_need_no_library(pkg, monkeypatch):
+    """The merged wrappers around plain modules, and what a CUDA-only module refuses, with no library built."""
+    monkeypatch.setattr(pkg._lib, "host", pkg._lib._Host())
+    monkeypatch.setattr(pkg._lib, "lib", lambda: (_ for _ in ()).throw(RuntimeError("no library")))
+    x = torch.randn(3, 8)
+    lin = [torch.nn.Linear(8, 8) for _ in range(3)]
+    for m in lin:
+        m.N = 8
+    assert torch.equal(pkg.SplitQKV(*lin)(x), torch.cat([m(x) for m in lin], dim=-1))
+    mlp = pkg.FusedPalettizedMLP(*lin, torch.nn.SiLU())
+    assert torch.allclose(mlp(x), lin[2](torch.nn.functional.silu(lin[0](x)) * lin[1](x)))
+    kg = pkg.KGroupedPalettizedLinear(torch.zeros(128 * 128 // 2, dtype=torch.uint8), torch.zeros(1, 128, 16).half(), 4, 128, 128)
+    with pytest.raises(RuntimeError, match="CUDA tensor"):
+        kg(torch.zeros(1, 128))
+    with pytest.raises(ValueError, match="feature dim"):
+        kg(torch.zeros(1, 64))
