@@ -5,6 +5,8 @@
 // here do the same work for the shapes and dtypes that need no conversion: look the module's native
 // description up, allocate the outputs, call the C entries. They return None, having launched
 // nothing, when a call is not one of those; the Python route then runs.
+#include <cstring>
+
 #include "merged.h"
 
 using namespace b200host;
@@ -52,16 +54,26 @@ static long int_of(PyObject* d, const char* key) {
   return v ? PyLong_AsLong(v) : 0;
 }
 
-// bind(module_dict, spec): spec is a dict with the layer's tensors and integers, "watch" (names in
-// the module whose objects it was built from) and "watch_params".
-static PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (n != 2 || !PyDict_Check(a[0]) || !PyDict_Check(a[1])) {
-    PyErr_SetString(PyExc_TypeError, "bind(module_dict, spec)");
-    return nullptr;
+static PyObject* g_library_error = nullptr;   // LibraryError(code, message) of the ctypes layer
+
+template <typename F>
+static PyObject* guarded(F&& f) {
+  try {
+    return f();
+  } catch (const LaunchError& e) {
+    if (!PyErr_Occurred()) {
+      PyObject* args = Py_BuildValue("(is)", e.code, e.what());
+      if (args) PyErr_SetObject(g_library_error ? g_library_error : PyExc_RuntimeError, args);
+      Py_XDECREF(args);
+    }
+  } catch (const std::exception& e) {
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
   }
-  PyObject *dict = a[0], *spec = a[1];
-  Layer* l = PyObject_New(Layer, &LayerType);
-  if (!l) return nullptr;
+  return nullptr;
+}
+
+// Fills `l` (zeroed) from the spec of bind(); null with an exception set, or a C++ exception, where it cannot.
+static PyObject* describe(Layer* l, PyObject* dict, PyObject* spec) {
   auto t = [&](const char* k) { return tensor_or_null(PyDict_GetItemString(spec, k)); };
   l->packed = t("packed"); l->lut = t("lut"); l->packed2 = t("packed2"); l->lut2 = t("lut2");
   l->bias = t("bias"); l->resA = t("resA"); l->resB = t("resB"); l->signs = t("signs"); l->awq = t("awq");
@@ -88,7 +100,7 @@ static PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
       return x.is_cuda() && x.scalar_type() == l->scalar && x.is_contiguous() &&
              (reinterpret_cast<uintptr_t>(x.const_data_ptr()) & 15) == 0;
     };
-    l->res_ok = A.size(1) <= 1024 && A.size(1) % 8 == 0 && fine(A) && fine(B);
+    l->res_ok = A.dim() == 2 && B.dim() == 2 && A.size(1) <= 1024 && A.size(1) % 8 == 0 && fine(A) && fine(B);
   }
   PyObject* names[2] = {PyDict_GetItemString(spec, "watch"), PyDict_GetItemString(spec, "watch_params")};
   for (int g = 0; g < 2; ++g) {
@@ -102,11 +114,23 @@ static PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
       l->watches->push_back(Watch{key, v, storage_of(v), g == 1});
     }
   }
-  if (PyErr_Occurred()) {
-    Py_DECREF(l);
+  return PyErr_Occurred() ? nullptr : reinterpret_cast<PyObject*>(l);
+}
+
+// bind(module_dict, spec): spec is a dict with the layer's tensors and integers, "watch" (names in
+// the module whose objects it was built from) and "watch_params".
+static PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 2 || !PyDict_Check(a[0]) || !PyDict_Check(a[1])) {
+    PyErr_SetString(PyExc_TypeError, "bind(module_dict, spec)");
     return nullptr;
   }
-  return reinterpret_cast<PyObject*>(l);
+  PyObject *dict = a[0], *spec = a[1];
+  Layer* l = PyObject_New(Layer, &LayerType);
+  if (!l) return nullptr;
+  std::memset(reinterpret_cast<char*>(l) + sizeof(PyObject), 0, sizeof(Layer) - sizeof(PyObject));
+  PyObject* done = guarded([&]() -> PyObject* { return describe(l, dict, spec); });
+  if (!done) Py_DECREF(l);
+  return done;
 }
 
 // ---- forwards ---------------------------------------------------------------------------------------
@@ -124,24 +148,6 @@ static at::Tensor output_like(const at::Tensor& x, int64_t cols, const Layer& l)
   c10::SmallVector<int64_t, 6> sizes(x.sizes().begin(), x.sizes().end());
   sizes.back() = cols;
   return empty(sizes, l.scalar, l.device);
-}
-
-static PyObject* g_library_error = nullptr;   // LibraryError(code, message) of the ctypes layer
-
-template <typename F>
-static PyObject* guarded(F&& f) {
-  try {
-    return f();
-  } catch (const LaunchError& e) {
-    if (!PyErr_Occurred()) {
-      PyObject* args = Py_BuildValue("(is)", e.code, e.what());
-      if (args) PyErr_SetObject(g_library_error ? g_library_error : PyExc_RuntimeError, args);
-      Py_XDECREF(args);
-    }
-  } catch (const std::exception& e) {
-    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
-  }
-  return nullptr;
 }
 
 static bool arguments(const char* what, PyObject* const* a, Py_ssize_t n) {

@@ -274,3 +274,28 @@ def test_modules_on_the_cpu_need_no_library(pkg, monkeypatch):
         kg(torch.zeros(1, 128))
     with pytest.raises(ValueError, match="feature dim"):
         kg(torch.zeros(1, 64))
+
+
+def test_a_description_that_cannot_be_built_raises(pkg):
+    """No C++ exception leaves the native host layer: a tensor without storage among what it looks at."""
+    import subprocess
+    import sys
+    code = """
+import importlib, sys
+sys.path.insert(0, %r)
+import torch
+pkg = importlib.import_module(%r)
+from torch._subclasses.fake_tensor import FakeTensorMode
+with FakeTensorMode():
+    fake = torch.empty(4, 4)
+for spec in (dict(N=128, K=128, lut2=fake, watch=("lut2",)),
+             dict(N=128, K=128, resA=torch.zeros(4), resB=torch.zeros(4))):
+    d = {"_buffers": {}, "_parameters": {}, **{k: v for k, v in spec.items() if k == "lut2"}}
+    try:
+        pkg._lib.host.bind(d, spec)
+    except Exception as e:
+        print("raised", type(e).__name__)
+print("alive")
+""" % (ROOT, pkg.__name__)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.splitlines()[-1] == "alive", r.stdout + r.stderr
