@@ -547,6 +547,14 @@ def _gemm_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     return host.workspace(device.index if device.index is not None else torch.cuda.current_device(), nbytes)
 
 
+def _gemm_workspace_need(M: int, N: int, K: int, s, flags: int) -> int:
+    """Scratch bytes that a launch over N output rows makes use of (CTA pairs are a form of the kernel that
+    takes the split schedule's workspace)."""
+    if flags & FLAG_CTA_PAIRS:
+        return lib().b200lut_gemm_workspace_bytes(M, N, K)
+    return lib().b200lut_gemm_launch_workspace_bytes(M, N, K, int(s.bits), int(s.group_size))
+
+
 def gemm(x: torch.Tensor, seg, epilogue: int = EPI_NONE, flags: int = 0, split: bool = True) -> None:
     """Prefill GEMM over one segment; brings the scratch buffer of the split schedule when the
     shape gains from it (split=False: whole-tile schedule)."""
@@ -558,7 +566,7 @@ def gemm(x: torch.Tensor, seg, epilogue: int = EPI_NONE, flags: int = 0, split: 
         if not split:
             flags |= FLAG_WHOLE_TILES
         elif not s0.packed2:
-            need = lib().b200lut_gemm_launch_workspace_bytes(M, int(s0.N), K, int(s0.bits), int(s0.group_size))
+            need = _gemm_workspace_need(M, int(s0.N), K, s0, flags)
         if need:
             ws = _gemm_workspace(x.device, need)
             check(lib().b200lut_gemm_ws(x.data_ptr(), x.stride(0), M, K, dtype_id(x.dtype), seg,
@@ -663,7 +671,7 @@ def gemm_multi(x: torch.Tensor, segs, nseg: int, flags: int = 0, split: bool = T
         total = sum(int(segs[i].N) for i in range(nseg))
         need = 0
         if split:
-            need = lib().b200lut_gemm_launch_workspace_bytes(M, total, K, int(segs[0].bits), int(segs[0].group_size))
+            need = _gemm_workspace_need(M, total, K, segs[0], flags)
         else:
             flags |= FLAG_WHOLE_TILES
         ws = _gemm_workspace(x.device, need) if need else None

@@ -391,3 +391,16 @@ def test_the_whole_tiles_flag_keeps_every_launch_from_cutting_k():
     one = {k: v for k, v in mod._segment_desc(want).items() if k not in ("packed2", "lut2", "bits2")}
     L.gemm(x, L.make_segments([one]), split=False)
     assert torch.equal(got, want)
+
+
+def test_cta_pairs_cut_the_tiles_of_the_last_round():
+    N, K, M = 1024, 2048, 300                    # eight tiles on 74 pairs of SMs
+    case = Case(N, K, 128, 4, torch.float16, seed=23)
+    mod = case.module()
+    mod._ensure_packed()
+    x = case.x(M).cuda()
+    outs = [torch.empty(M, N, dtype=torch.float16, device="cuda") for _ in range(2)]
+    for out, split in zip(outs, (True, False)):
+        L.gemm(x, L.make_segments([mod._segment_desc(out)]), flags=L.FLAG_CTA_PAIRS, split=split)
+    assert rel_err(outs[0], outs[1]) <= 2.0 ** -10       # neighbouring fp16 values
+    assert not torch.equal(outs[0], outs[1])             # sums in parts
