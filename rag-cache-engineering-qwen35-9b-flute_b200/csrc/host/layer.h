@@ -11,8 +11,10 @@
 
 #include <ATen/ATen.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
+#include <string>
 #include <vector>
 
 #include "../../../include/b200_lut.h"
@@ -94,9 +96,14 @@ inline PyObject* child_dict(PyObject* dict, PyObject* name, PyObject** child = n
   return d;
 }
 
+// The Python route's rule: "1", "true" or "True", whitespace around it aside.
 inline bool env_on(const char* name) {
   const char* e = std::getenv(name);
-  return e && (e[0] == '1' || e[0] == 't' || e[0] == 'T');
+  if (!e) return false;
+  std::string v(e);
+  v.erase(0, std::min(v.find_first_not_of(" \t\r\n\v\f"), v.size()));
+  v.erase(v.find_last_not_of(" \t\r\n\v\f") + 1);
+  return v == "1" || v == "true" || v == "True";
 }
 
 }  // namespace b200host

@@ -164,3 +164,13 @@ def test_a_residual_factor_written_in_place_is_followed(which):
         m.resB.mul_(-3)
     want = other(x)                                         # stacked after the change
     assert torch.equal(mod(x), want) and torch.equal(mod._forward_route(x), want) and torch.equal(mod(x), want)
+
+
+@pytest.mark.parametrize("value,off", ((" 1 ", True), ("true", True), ("True\n", True), ("TRUE", False), ("10", False), ("", False)))
+def test_the_merge_switch_reads_as_in_the_python_route(value, off, monkeypatch):
+    mk = lambda n, s: Case(n, 256, 128, 4, torch.bfloat16, seed=s).module()     # noqa: E731
+    qkv = pkg.SplitQKV(mk(256, 1), mk(128, 2), mk(128, 3))
+    x = torch.randn(4, 256, device="cuda").bfloat16()
+    qkv(x), qkv(x)
+    monkeypatch.setenv("FLUTE_NO_MERGE", value)
+    assert (pkg._lib.host.qkv(qkv.__dict__, x, True) is None) == off
