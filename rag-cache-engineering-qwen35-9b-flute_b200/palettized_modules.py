@@ -876,6 +876,7 @@ class PalettizedEmbedding(nn.Module):
         self._packed2 = None
         self._tied = []          # [PalettizedLinear] whose slab copies serve this table
         self._bad_ids = None     # device flag: a forward met a CUDA id outside [0, N)
+        self._bad_id_flag()
 
     @classmethod
     def tied_to(cls, lm: PalettizedLinear) -> "PalettizedEmbedding":
@@ -902,6 +903,7 @@ class PalettizedEmbedding(nn.Module):
             emb.rot_signs, emb._signs_cache = lm.rot_signs, {}
             emb._packed = emb._packed2 = None
             emb._bad_ids = None
+            emb._bad_id_flag()
         emb._tied = [lm]
         return emb
 
@@ -988,12 +990,21 @@ class PalettizedEmbedding(nn.Module):
                            "bitwidth2", "group_size", "rot_signs"))
         self.__dict__["_native"] = _lib.host.bind(self.__dict__, spec)
 
-    def _bad_id_flag(self) -> torch.Tensor:
-        """Device word that a gather sets when it meets an id outside [0, N)."""
+    def _bad_id_flag(self) -> Optional[torch.Tensor]:
+        """Device word that a gather sets when it meets an id outside [0, N). It is made when the table
+        comes to a device, not in a forward that may be under stream capture: a graph would own the word
+        and clear it in every replay."""
+        if not self.lut.is_cuda:
+            return None
         flag = self.__dict__.get("_bad_id_word")
         if flag is None or flag.device != self.lut.device:
             flag = self.__dict__["_bad_id_word"] = torch.zeros(1, dtype=torch.int32, device=self.lut.device)
         return flag
+
+    def _apply(self, fn, *args, **kwargs):
+        super()._apply(fn, *args, **kwargs)
+        self._bad_id_flag()
+        return self
 
     def forward(self, ids):
         native = self.__dict__.get("_native")

@@ -180,3 +180,29 @@ def test_cuda_ids_out_of_range_are_zero_rows_and_reported():
     assert pkg._lib.lib().b200lut_device_status() == 0
     with pytest.raises(ValueError, match="out of range"):
         emb(torch.tensor([N]))
+
+
+def test_a_graph_replay_keeps_what_eager_gathers_recorded():
+    """The first gather of a table under stream capture: the word that records a bad id is the module's, not
+    the graph's, so a replay with good ids does not clear what an eager gather recorded."""
+    lut = torch.randn(2, 16, generator=torch.Generator().manual_seed(4)).half()
+    blob = torch.randint(0, 256, (256 * 128 // 2,), dtype=torch.uint8)
+    emb = pkg.PalettizedEmbedding(blob, lut, 4, 128, 256, 128).cuda()
+    emb._table()                                               # codes repacked; no gather yet
+    ids = torch.arange(8, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = emb(ids)
+    g.replay()
+    assert torch.equal(out, emb(ids))
+    emb.check_ids()
+    emb(torch.full((3,), 256, device="cuda"))
+    g.replay()
+    with pytest.raises(ValueError, match="out of range"):
+        emb.check_ids()
+    assert pkg._lib.lib().b200lut_device_status() == 0
+    ids.fill_(-1)                                              # and a replay records its own
+    emb(torch.zeros(1, dtype=torch.int64, device="cuda"))
+    g.replay()
+    with pytest.raises(ValueError, match="out of range"):
+        emb.check_ids()
