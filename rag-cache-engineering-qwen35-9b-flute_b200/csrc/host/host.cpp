@@ -20,6 +20,7 @@ static void layer_clear(Layer* l) {
     for (Watch& w : *l->watches) {
       Py_XDECREF(w.key);
       Py_XDECREF(w.value);
+      Py_XDECREF(w.dict);
     }
     delete l->watches;
   }
@@ -102,23 +103,28 @@ static PyObject* describe(Layer* l, PyObject* dict, PyObject* spec) {
     };
     l->res_ok = A.dim() == 2 && B.dim() == 2 && A.size(1) <= 1024 && A.size(1) % 8 == 0 && fine(A) && fine(B);
   }
-  PyObject* names[2] = {PyDict_GetItemString(spec, "watch"), PyDict_GetItemString(spec, "watch_params")};
-  for (int g = 0; g < 2; ++g) {
+  PyObject* tied = PyDict_GetItemString(spec, "tied");
+  PyObject* names[3] = {PyDict_GetItemString(spec, "watch"), PyDict_GetItemString(spec, "watch_params"),
+                        tied ? PyDict_GetItemString(spec, "watch_tied") : nullptr};
+  for (int g = 0; g < 3; ++g) {
     if (!names[g]) continue;
     for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(names[g]); ++i) {
       PyObject* key = PyTuple_GET_ITEM(names[g], i);
       Py_INCREF(key);
       PyUnicode_InternInPlace(&key);
-      PyObject* v = lookup(dict, key, g == 1);
+      PyObject* v = lookup(g == 2 ? tied : dict, key, g == 1);
       Py_XINCREF(v);
-      l->watches->push_back(Watch{key, v, storage_of(v), g == 1});
+      if (g == 2) Py_INCREF(tied);
+      l->watches->push_back(Watch{key, v, g == 2 ? tied : nullptr, g == 1, v && THPVariable_Check(v), Look()});
+      if (l->watches->back().tensor) l->watches->back().look = look_of(THPVariable_Unpack(v));
     }
   }
   return PyErr_Occurred() ? nullptr : reinterpret_cast<PyObject*>(l);
 }
 
 // bind(module_dict, spec): spec is a dict with the layer's tensors and integers, "watch" (names in
-// the module whose objects it was built from) and "watch_params".
+// the module whose objects it was built from) and "watch_params"; "tied" and "watch_tied" name what
+// belongs to another module, by its __dict__.
 static PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 2 || !PyDict_Check(a[0]) || !PyDict_Check(a[1])) {
     PyErr_SetString(PyExc_TypeError, "bind(module_dict, spec)");

@@ -1,9 +1,9 @@
 // Native description of one palettized projection, kept in its module's __dict__ as "_native".
 //
-// The module stays the owner of its state: a description remembers which objects (and which
-// storage) it was built from and is only used while the module still holds exactly those, so
-// .to(), drop_blob(), a replaced palette or a changed option all lead back to the Python route,
-// which builds a new one.
+// The module stays the owner of its state: a description remembers which objects it was built from and
+// what its tensors looked like (storage, type, shape), and is only used while the module still holds
+// exactly those, so .to(), drop_blob(), a replaced palette or a changed option all lead back to the
+// Python route, which builds a new one.
 #pragma once
 
 #include <Python.h>
@@ -21,12 +21,22 @@
 
 namespace b200host {
 
-// One entry of the module that the description depends on.
+// What a tensor looks like from outside: its address, type, sizes and strides. A tensor can change all of
+// them and stay the same object (set_, t_, an assignment to .data).
+struct Look {
+  const void* data = nullptr;
+  at::ScalarType type = at::kFloat;
+  c10::SmallVector<int64_t, 4> sizes, strides;
+};
+
+// One entry of the module (or of the module it is tied to) that the description depends on.
 struct Watch {
   PyObject* key;        // interned name
   PyObject* value;      // the object found under it when the description was built, or null
-  const void* data;     // a tensor's storage address (null for other objects)
+  PyObject* dict;       // the other module's __dict__, or null: the module's own
   bool in_params;       // looked up in _parameters instead of _buffers / __dict__
+  bool tensor;
+  Look look;
 };
 
 struct Layer {
@@ -56,15 +66,25 @@ inline PyObject* lookup(PyObject* dict, PyObject* key, bool in_params) {
   return PyDict_GetItemWithError(dict, key);
 }
 
-inline const void* storage_of(PyObject* o) {
-  return o && THPVariable_Check(o) ? THPVariable_Unpack(o).const_data_ptr() : nullptr;
+inline Look look_of(const at::Tensor& t) {
+  Look l;
+  l.data = t.const_data_ptr();
+  l.type = t.scalar_type();
+  l.sizes.assign(t.sizes().begin(), t.sizes().end());
+  l.strides.assign(t.strides().begin(), t.strides().end());
+  return l;
+}
+
+inline bool looks_the_same(const at::Tensor& t, const Look& l) {
+  return t.const_data_ptr() == l.data && t.scalar_type() == l.type && t.sizes() == at::IntArrayRef(l.sizes) &&
+         t.strides() == at::IntArrayRef(l.strides);
 }
 
 inline bool current(const Layer& l, PyObject* dict) {
   for (const Watch& w : *l.watches) {
-    PyObject* v = lookup(dict, w.key, w.in_params);
+    PyObject* v = lookup(w.dict ? w.dict : dict, w.key, w.in_params);
     if (v != w.value) return false;
-    if (w.data && storage_of(v) != w.data) return false;
+    if (w.tensor && !looks_the_same(THPVariable_Unpack(v), w.look)) return false;
   }
   return true;
 }

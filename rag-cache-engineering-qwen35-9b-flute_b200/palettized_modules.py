@@ -988,6 +988,8 @@ class PalettizedEmbedding(nn.Module):
                     group_size=self.group_size, n_groups=self.lut.shape[0],
                     watch=("lut", "lut2", "resA", "resB", "indices2", "_packed", "_packed2", "_tied", "N", "K", "bitwidth",
                            "bitwidth2", "group_size", "rot_signs"))
+        if self._tied:       # the codes are the head's
+            spec.update(tied=self._tied[0].__dict__, watch_tied=("_packed", "_packed2", "lut"))
         self.__dict__["_native"] = _lib.host.bind(self.__dict__, spec)
 
     def _bad_id_flag(self) -> Optional[torch.Tensor]:

@@ -174,3 +174,25 @@ def test_the_merge_switch_reads_as_in_the_python_route(value, off, monkeypatch):
     qkv(x), qkv(x)
     monkeypatch.setenv("FLUTE_NO_MERGE", value)
     assert (pkg._lib.host.qkv(qkv.__dict__, x, True) is None) == off
+
+
+def test_a_tensor_changed_in_place_is_described_anew():
+    case = Case(256, 128, 128, 4, torch.float16, seed=31, residual=128)     # a square second factor
+    mod = case.module()
+    x = case.x(3).cuda()
+    mod(x), mod(x)
+    mod.resB.t_()                                           # same object, same storage, other strides
+    case.resB = case.resB.t().contiguous()
+    assert rel_err(mod(x), case.oracle(case.x(3))) <= TOL
+
+
+def test_a_tied_table_follows_the_codes_of_its_head():
+    head, other = (Case(256, 128, 128, 4, torch.bfloat16, seed=s) for s in (32, 33))
+    lm = head.module()
+    emb = pkg.PalettizedEmbedding.tied_to(lm).cuda()
+    ids = torch.arange(256, device="cuda")
+    emb(ids), emb(ids)
+    lm.indices, lm._packed = other.blob.cuda(), None        # new codes under the same palettes
+    want = other.codes.astype("int64")
+    pal = head.lut.float()[torch.arange(256) // 128]
+    assert torch.equal(emb(ids).float().cpu(), pal.gather(1, torch.from_numpy(want)))
