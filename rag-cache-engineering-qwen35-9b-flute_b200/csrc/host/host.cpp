@@ -172,8 +172,14 @@ static PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Ctx c;
     if (!l || !rows_of(x, *l, &r) || linear_kind(*l, r.M) == Kind::kNotServed || !context(l->device, a[2] == Py_True, &c))
       Py_RETURN_NONE;
-    at::Tensor out = output_like(x, l->N, *l);
-    linear_into(*l, r, out.mutable_data_ptr(), l->N, c);
+    const bool fused = rotation_fuses(*l, r.M);
+    const Held held(l);
+    at::Tensor out;
+    {
+      const WithoutGil free;
+      out = output_like(x, l->N, *l);
+      linear_into(*l, r, out.mutable_data_ptr(), l->N, fused, c);
+    }
     return THPVariable_Wrap(std::move(out));
   });
 }
@@ -197,11 +203,18 @@ static PyObject* qkv(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Rows r;
     Ctx c;
     if (!rows_of(x, *ls[0], &r) || !mergeable(a[0], ls, 3, r.M) || !context(ls[0]->device, a[2] == Py_True, &c)) Py_RETURN_NONE;
-    at::Tensor out = output_like(x, total, *ls[0]);
-    char* p = static_cast<char*>(out.mutable_data_ptr());
-    void* outs[3];
-    for (int i = 0; i < 3; p += 2 * int64_t(ls[i]->N), ++i) outs[i] = p;
-    merged_into(a[0], ls, 3, r, outs, total, B200LUT_EPI_NONE, c);
+    const bool fused = merged_rotation_fuses(ls, 3, r.M);
+    const at::Tensor stack = stack_or_none(a[0], ls, 3, r.M);
+    const Held h0(ls[0]), h1(ls[1]), h2(ls[2]);
+    at::Tensor out;
+    {
+      const WithoutGil free;
+      out = output_like(x, total, *ls[0]);
+      char* p = static_cast<char*>(out.mutable_data_ptr());
+      void* outs[3];
+      for (int i = 0; i < 3; p += 2 * int64_t(ls[i]->N), ++i) outs[i] = p;
+      merged_into(stack, ls, 3, r, outs, total, B200LUT_EPI_NONE, fused, c);
+    }
     return THPVariable_Wrap(std::move(out));
   });
 }
@@ -228,16 +241,23 @@ static PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
         down.device != ls[0]->device || !mergeable(a[0], ls, 2, r.M) || linear_kind(down, r.M) == Kind::kNotServed ||
         !context(down.device, a[2] == Py_True, &c))
       Py_RETURN_NONE;
-    at::Tensor g = empty({r.M, I}, down.scalar, down.device), u;
-    void* outs[2] = {g.mutable_data_ptr(), nullptr};
-    if (r.M > kGemvMaxM) {
-      u = empty({r.M, I}, down.scalar, down.device);
-      outs[1] = u.mutable_data_ptr();
+    const bool fused = merged_rotation_fuses(ls, 2, r.M), down_fused = rotation_fuses(down, r.M);
+    const at::Tensor stack = stack_or_none(a[0], ls, 2, r.M);
+    const Held h0(ls[0]), h1(ls[1]), h2(ls[2]);
+    at::Tensor out;
+    {
+      const WithoutGil free;
+      at::Tensor g = empty({r.M, I}, down.scalar, down.device), u;
+      void* outs[2] = {g.mutable_data_ptr(), nullptr};
+      if (r.M > kGemvMaxM) {
+        u = empty({r.M, I}, down.scalar, down.device);
+        outs[1] = u.mutable_data_ptr();
+      }
+      merged_into(stack, ls, 2, r, outs, I, r.M > kGemvMaxM ? B200LUT_EPI_NONE : B200LUT_EPI_SILU_MUL, fused, c);
+      if (r.M > kGemvMaxM) check(b200lut_silu_mul(outs[0], outs[1], r.M, I, I, I, down.dtype, c.stream));
+      out = output_like(x, down.N, down);
+      linear_into(down, Rows{outs[0], I, r.M}, out.mutable_data_ptr(), down.N, down_fused, c);
     }
-    merged_into(a[0], ls, 2, r, outs, I, r.M > kGemvMaxM ? B200LUT_EPI_NONE : B200LUT_EPI_SILU_MUL, c);
-    if (r.M > kGemvMaxM) check(b200lut_silu_mul(outs[0], outs[1], r.M, I, I, I, down.dtype, c.stream));
-    at::Tensor out = output_like(x, down.N, down);
-    linear_into(down, Rows{outs[0], I, r.M}, out.mutable_data_ptr(), down.N, c);
     return THPVariable_Wrap(std::move(out));
   });
 }
@@ -251,23 +271,29 @@ static PyObject* kgrouped(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Rows r;
     Ctx c;
     if (!l || !l->kgrouped || !rows_of(x, *l, &r) || !context(l->device, a[2] == Py_True, &c)) Py_RETURN_NONE;
-    at::Tensor out = output_like(x, l->N, *l);
-    const void* bias = l->bias ? l->bias->const_data_ptr() : nullptr;
-    if (r.M <= kGemvMaxM) {
-      // without a scratch the entry refuses the shapes that need one: the Python route brings it
-      const int rc = b200lut_gemv_kgrouped(r.ptr, r.ld, r.M, l->K, l->dtype, l->packed->const_data_ptr(),
-                                           l->lut->const_data_ptr(), bias, l->N, l->bits, out.mutable_data_ptr(), l->N, 0,
-                                           nullptr, 0, c.stream);
-      if (rc == B200LUT_ERR_WORKSPACE) Py_RETURN_NONE;
-      check(rc);
-    } else {
-      const size_t need = b200lut_gemm_workspace_bytes(r.M, l->N, l->K);
-      at::Tensor ws;
-      if (need) ws = scratch_pool().get(Scratch::kSplit, c.device, c.stream, need);
-      check(b200lut_gemm_kgrouped(r.ptr, r.ld, r.M, l->K, l->dtype, l->packed->const_data_ptr(), l->lut->const_data_ptr(),
-                                  bias, l->N, l->bits, out.mutable_data_ptr(), l->N, c.flags,
-                                  need ? ws.mutable_data_ptr() : nullptr, need ? size_t(ws.numel()) : 0, c.stream));
+    const Held held(l);
+    at::Tensor out;
+    {
+      const WithoutGil free;
+      out = output_like(x, l->N, *l);
+      const void* bias = l->bias ? l->bias->const_data_ptr() : nullptr;
+      if (r.M <= kGemvMaxM) {
+        // without a scratch the entry refuses the shapes that need one: the Python route brings it
+        const int rc = b200lut_gemv_kgrouped(r.ptr, r.ld, r.M, l->K, l->dtype, l->packed->const_data_ptr(),
+                                             l->lut->const_data_ptr(), bias, l->N, l->bits, out.mutable_data_ptr(), l->N, 0,
+                                             nullptr, 0, c.stream);
+        if (rc == B200LUT_ERR_WORKSPACE) out.reset();
+        else check(rc);
+      } else {
+        const size_t need = b200lut_gemm_workspace_bytes(r.M, l->N, l->K);
+        at::Tensor ws;
+        if (need) ws = scratch_pool().get(Scratch::kSplit, c.device, c.stream, need);
+        check(b200lut_gemm_kgrouped(r.ptr, r.ld, r.M, l->K, l->dtype, l->packed->const_data_ptr(), l->lut->const_data_ptr(),
+                                    bias, l->N, l->bits, out.mutable_data_ptr(), l->N, c.flags,
+                                    need ? ws.mutable_data_ptr() : nullptr, need ? size_t(ws.numel()) : 0, c.stream));
+      }
     }
+    if (!out.defined()) Py_RETURN_NONE;
     return THPVariable_Wrap(std::move(out));
   });
 }
@@ -285,15 +311,20 @@ static PyObject* embed(PyObject*, PyObject* const* a, Py_ssize_t n) {
       Py_RETURN_NONE;
     c10::SmallVector<int64_t, 6> sizes(ids.sizes().begin(), ids.sizes().end());
     sizes.push_back(l->K);
-    at::Tensor out = empty(sizes, l->scalar, l->device);
-    b200lut_segment s = segment(*l, out.mutable_data_ptr(), l->K);
-    if (l->res) {
-      s.resA = l->resA->const_data_ptr();
-      s.res_rank = int(l->resA->size(1));
+    const Held held(l);
+    at::Tensor out;
+    {
+      const WithoutGil free;
+      out = empty(sizes, l->scalar, l->device);
+      b200lut_segment s = segment(*l, out.mutable_data_ptr(), l->K);
+      if (l->res) {
+        s.resA = l->resA->const_data_ptr();
+        s.res_rank = int(l->resA->size(1));
+      }
+      check(b200lut_embed_gather_checked(ids.const_data_ptr<int64_t>(), ids.numel(), l->K, l->dtype, &s,
+                                         l->res ? l->resB->const_data_ptr() : nullptr, 0,
+                                         static_cast<int32_t*>(bad.mutable_data_ptr()), c.stream));
     }
-    check(b200lut_embed_gather_checked(ids.const_data_ptr<int64_t>(), ids.numel(), l->K, l->dtype, &s,
-                                       l->res ? l->resB->const_data_ptr() : nullptr, 0,
-                                       static_cast<int32_t*>(bad.mutable_data_ptr()), c.stream));
     return THPVariable_Wrap(std::move(out));
   });
 }
@@ -328,9 +359,13 @@ static PyObject* fht(PyObject*, PyObject* const* a, Py_ssize_t n) {
         Py_RETURN_NONE;
       v[i] = static_cast<const float*>(t.const_data_ptr());
     }
-    at::Tensor y = empty(x.sizes(), x.scalar_type(), c.device);
-    check(b200lut_fht(x.const_data_ptr(), y.mutable_data_ptr(), v[0], v[1], int(M), int(K), K, K, dtype, int(mode),
-                      int(block), c.stream));
+    at::Tensor y;
+    {
+      const WithoutGil free;
+      y = empty(x.sizes(), x.scalar_type(), c.device);
+      check(b200lut_fht(x.const_data_ptr(), y.mutable_data_ptr(), v[0], v[1], int(M), int(K), K, K, dtype, int(mode),
+                        int(block), c.stream));
+    }
     return THPVariable_Wrap(std::move(y));
   });
 }
@@ -346,7 +381,11 @@ static PyObject* workspace(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (PyErr_Occurred()) return nullptr;
   return guarded([&]() -> PyObject* {
     const cudaStream_t st = c10::cuda::getCurrentCUDAStream(c10::DeviceIndex(device)).stream();
-    at::Tensor t = scratch_pool().get(Scratch::kSplit, int(device), st, bytes);
+    at::Tensor t;
+    {
+      const WithoutGil free;      // the pool's lock is only ever taken without the interpreter's
+      t = scratch_pool().get(Scratch::kSplit, int(device), st, bytes);
+    }
     return THPVariable_Wrap(std::move(t));
   });
 }

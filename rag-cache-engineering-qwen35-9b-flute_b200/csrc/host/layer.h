@@ -104,6 +104,20 @@ inline Layer* layer_of(PyObject* dict) {
   return l;
 }
 
+// Lets other Python threads run while this one allocates and launches (a launch blocks when the stream's
+// queue is full, and what drains the queue may be a host function that needs the interpreter). Whatever
+// the launches use is held by the caller: layers by Held, tensors by reference.
+struct WithoutGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+struct Held {
+  PyObject* o;
+  explicit Held(void* p) : o(static_cast<PyObject*>(p)) { Py_XINCREF(o); }
+  ~Held() { Py_XDECREF(o); }
+  Held(const Held&) = delete;
+};
+
 // Child module `name` of a module's __dict__: its own __dict__ (borrowed), or null.
 inline PyObject* child_dict(PyObject* dict, PyObject* name, PyObject** child = nullptr) {
   PyObject* mods = PyDict_GetItemWithError(dict, name_modules());

@@ -37,6 +37,13 @@ inline const at::Tensor* residual_stack(PyObject* owner_dict, Layer* const* ls, 
   return at_factor == PyTuple_GET_SIZE(factors) ? &THPVariable_Unpack(stack) : nullptr;
 }
 
+// The stack that a launch of M rows reads, undefined where there is none to read.
+inline at::Tensor stack_or_none(PyObject* owner_dict, Layer* const* ls, int n, int M) {
+  bool any_res = false;
+  for (int i = 0; i < n; ++i) any_res = any_res || ls[i]->res;
+  return any_res && M <= kGemvMaxM ? *residual_stack(owner_dict, ls, n) : at::Tensor();
+}
+
 inline bool same_fold(const Layer& a, const Layer& b) {
   if (!a.rotated || !b.rotated) return !a.rotated && !b.rotated;
   return a.rotation && b.rotation && PyObject_RichCompareBool(a.rotation, b.rotation, Py_EQ) == 1;
@@ -57,16 +64,20 @@ inline bool mergeable(PyObject* owner_dict, Layer* const* ls, int n, int M) {
   return !any_res || M > kGemvMaxM || residual_stack(owner_dict, ls, n) != nullptr;
 }
 
+inline bool merged_rotation_fuses(Layer* const* ls, int n, int M) {
+  bool fused = ls[0]->rotated;
+  for (int i = 0; i < n; ++i) fused = fused && rotation_fuses(*ls[i], M);
+  return fused;
+}
+
 // The merged launch into outs[i] (row stride ld): M <= 16 the decode kernels, with EPI_SILU_MUL only
 // outs[0] is written; M > 16 the tensor-core GEMM (no epilogue there).
-inline void merged_into(PyObject* owner_dict, Layer* const* ls, int n, Rows r, void* const* outs, int64_t ld, int epilogue,
-                        const Ctx& c) {
+// `fused` is merged_rotation_fuses(), `stack` the residual_stack() of M <= 16. Runs without the interpreter lock.
+inline void merged_into(const at::Tensor& stack, Layer* const* ls, int n, Rows r, void* const* outs, int64_t ld, int epilogue,
+                        bool fused, const Ctx& c) {
   const Layer& a = *ls[0];
-  bool fused = a.rotated, any_res = false;
-  for (int i = 0; i < n; ++i) {
-    fused = fused && rotation_fuses(*ls[i], r.M);
-    any_res = any_res || ls[i]->res;
-  }
+  bool any_res = false;
+  for (int i = 0; i < n; ++i) any_res = any_res || ls[i]->res;
   at::Tensor rotated, t;
   if (a.rotated && !fused) {
     rotated = rotate(a, r, c);
@@ -80,7 +91,6 @@ inline void merged_into(PyObject* owner_dict, Layer* const* ls, int n, Rows r, v
   }
   if (r.M <= kGemvMaxM) {
     if (any_res) {
-      const at::Tensor& stack = *residual_stack(owner_dict, ls, n);
       const int cols = int(stack.size(0));
       t = empty({r.M, cols}, at::kFloat, c.device);
       float* tp = static_cast<float*>(t.mutable_data_ptr());

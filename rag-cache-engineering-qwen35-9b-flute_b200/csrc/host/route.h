@@ -138,10 +138,10 @@ inline void gemm_launch(const Rows& r, int K, int dtype, const b200lut_segment* 
   else check(b200lut_gemm_multi(r.ptr, r.ld, r.M, K, dtype, segs, n, c.flags, wp, wb, c.stream));
 }
 
-// out[M, N] (row stride ldo) = the layer on rows r; linear_kind() has said it is served.
-inline void linear_into(const Layer& l, Rows r, void* out, int64_t ldo, const Ctx& c) {
+// out[M, N] (row stride ldo) = the layer on rows r; linear_kind() has said it is served, `fused` is
+// rotation_fuses(). Runs without the interpreter lock.
+inline void linear_into(const Layer& l, Rows r, void* out, int64_t ldo, bool fused, const Ctx& c) {
   const Kind kind = linear_kind(l, r.M);
-  const bool fused = rotation_fuses(l, r.M);
   at::Tensor rotated, t;
   if (l.rotated && !fused) {
     rotated = rotate(l, r, c);

@@ -196,3 +196,35 @@ def test_a_tied_table_follows_the_codes_of_its_head():
     want = other.codes.astype("int64")
     pal = head.lut.float()[torch.arange(256) // 128]
     assert torch.equal(emb(ids).float().cpu(), pal.gather(1, torch.from_numpy(want)))
+
+
+def test_other_python_threads_run_while_a_launch_waits_for_room_in_the_queue():
+    # the device sleeps for a quarter of a second; the launches behind it fill the stream's queue and block
+    import threading
+    import time
+    case = Case(128, 128, 128, 4, torch.bfloat16, seed=41)
+    mod = case.module()
+    x = case.x(1).cuda()
+    mod(x), mod(x)
+    torch.cuda.synchronize()
+    gaps, stop = [], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+    t = threading.Thread(target=tick)
+    t.start()
+    t0 = time.perf_counter()
+    torch.cuda._sleep(500_000_000)
+    for _ in range(8000):
+        mod(x)
+    blocked = time.perf_counter() - t0
+    stop.set()
+    t.join()
+    torch.cuda.synchronize()
+    assert blocked > 0.1, "the queue never filled"
+    assert max(gaps) < 0.08
