@@ -10,6 +10,7 @@ from __future__ import annotations
 import ctypes
 import importlib.util
 import os
+import threading
 from typing import Optional, Sequence
 
 import torch
@@ -538,6 +539,7 @@ def round_rows(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
 
 
 _gemm_scratch = {}
+_two_stream_launches = threading.Lock()
 
 
 def _gemm_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
@@ -645,8 +647,9 @@ def gemm_two_stream(x: torch.Tensor, seg, flags: int = 0) -> None:
             buf = torch.empty(max(need, 2 * buf.numel() if buf is not None else 0), dtype=torch.uint8,
                               device=x.device)
             _gemm_scratch[key] = buf
-        check(lib().b200lut_gemm_two_stream(x.data_ptr(), x.stride(0), M, K, dtype_id(x.dtype), seg, flags,
-                                            buf.data_ptr(), buf.numel(), _stream(x)))
+        with _two_stream_launches:      # two launches share the scratch: no other thread's between them
+            check(lib().b200lut_gemm_two_stream(x.data_ptr(), x.stride(0), M, K, dtype_id(x.dtype), seg, flags,
+                                                buf.data_ptr(), buf.numel(), _stream(x)))
 
 
 GEMM_MULTI_MAX = 4

@@ -176,6 +176,8 @@ inline void linear_into(const Layer& l, Rows r, void* out, int64_t ldo, bool fus
   } else {
     const size_t need = b200lut_gemm_two_stream_bytes(r.M, l.N);
     at::Tensor ws = scratch_pool().get(Scratch::kTwoStream, c.device, c.stream, need);
+    // two launches that share the scratch: another thread's on this stream must not come between them
+    const std::lock_guard<std::mutex> both(scratch_pool().two_stream_launches());
     check(b200lut_gemm_two_stream(r.ptr, r.ld, r.M, l.K, l.dtype, &s, c.flags, ws.mutable_data_ptr(),
                                   size_t(ws.numel()), c.stream));
   }

@@ -43,6 +43,8 @@ class ScratchPool {
     return buf;
   }
 
+  std::mutex& two_stream_launches() { return two_stream_; }
+
  private:
   static constexpr size_t kMaxEntries = 32;
   struct Entry {
@@ -52,7 +54,7 @@ class ScratchPool {
     unsigned long long capture;
     at::Tensor buf;
   };
-  std::mutex mu_;
+  std::mutex mu_, two_stream_;
   std::list<Entry> entries_;
 };
 

@@ -228,3 +228,24 @@ def test_other_python_threads_run_while_a_launch_waits_for_room_in_the_queue():
     torch.cuda.synchronize()
     assert blocked > 0.1, "the queue never filled"
     assert max(gaps) < 0.08
+
+
+def test_threads_of_one_stream_do_not_mix_their_two_stream_launches():
+    import threading
+    mods = [Case(256, 256, 128, 4, torch.float16, seed=s, bits2=2).module() for s in (51, 52)]
+    x = torch.randn(40, 256, device="cuda").half()
+    wants = [m(x) for m in mods]
+    assert all(pkg._lib.host.linear(m.__dict__, x, True) is not None for m in mods)
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        outs = [mods[i](x) for _ in range(1500)]
+        torch.cuda.synchronize()
+        bad.append(sum(not torch.equal(o, wants[i]) for o in outs))
+    threads = [threading.Thread(target=work, args=(i % 2,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert bad == [0] * 4
