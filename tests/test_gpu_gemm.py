@@ -404,3 +404,61 @@ def test_cta_pairs_cut_the_tiles_of_the_last_round():
         L.gemm(x, L.make_segments([mod._segment_desc(out)]), flags=L.FLAG_CTA_PAIRS, split=split)
     assert rel_err(outs[0], outs[1]) <= 2.0 ** -10       # neighbouring fp16 values
     assert not torch.equal(outs[0], outs[1])             # sums in parts
+
+
+# ---- the persistent kernel's split schedule: more rows than the kernel for short prompts takes ------------
+
+@pytest.mark.parametrize("N,K,gs,bits,dtype,M,bias,residual", (
+    (1280, 512, 128, 4, torch.bfloat16, 1100, True, 0),      # 50 tiles, cut in two
+    (512, 1024, 64, 4, torch.float16, 1025, False, 0),       # a token tile of one row
+    (512, 1024, 128, 2, torch.bfloat16, 1200, True, 0),      # 20 tiles, cut in seven
+    (640, 1088, 128, 4, torch.float16, 1024, True, 40),      # residual k-blocks in the last part
+    (4096, 256, 64, 3, torch.bfloat16, 1300, False, 0),      # 192 tiles: a whole round and 44 cut ones
+))
+def test_split_schedule_beyond_short_prompts(N, K, gs, bits, dtype, M, bias, residual):
+    assert L.lib().b200lut_gemm_launch_workspace_bytes(M, N, K, bits, gs) > 0
+    case = Case(N, K, gs, bits, dtype, seed=N + M, bias=bias, residual=residual)
+    mod = case.module()
+    x = case.x(M)
+    want = case.oracle(x)
+    first = mod(x.cuda())
+    assert rel_err(first, want) <= TOL
+    assert torch.equal(mod(x.cuda()), first)                 # the counters returned to zero by themselves
+    t = L.residual_project_rows(x.cuda(), mod.resB) if residual else None
+    for split in (True, False):
+        buf = torch.full((M, N + 24), 7.0, dtype=dtype, device="cuda")
+        view = buf[:, 3:3 + N]                               # 6 bytes off the 16-byte grid, row stride N + 24
+        L.gemm(x.cuda(), L.make_segments([mod._segment_desc(view, ldo=N + 24, res_t=t)]), split=split)
+        assert rel_err(view, want) <= TOL
+        assert (buf[:, :3] == 7.0).all() and (buf[:, 3 + N:] == 7.0).all()
+
+
+def test_a_workspace_the_split_schedule_cannot_use_is_not_touched():
+    N, K, M = 1280, 512, 1100
+    case = Case(N, K, 128, 4, torch.bfloat16, seed=6)
+    mod = case.module()
+    mod._ensure_packed()
+    x = case.x(M).cuda()
+    whole = _raw_gemm(case, mod, x, split=False)
+    need = L.lib().b200lut_gemm_launch_workspace_bytes(M, N, K, 4, 128)
+    assert need > 0
+    ws = torch.zeros(need + 16, dtype=torch.uint8, device="cuda")
+    out = torch.empty_like(whole)
+    seg = L.make_segments([mod._segment_desc(out)])
+    for ptr, size, used in ((ws.data_ptr(), need - 1, False), (ws.data_ptr() + 4, need, False), (ws.data_ptr(), need, True)):
+        out.zero_()
+        L.check(L.lib().b200lut_gemm_ws(x.data_ptr(), x.stride(0), M, K, L.dtype_id(x.dtype), seg,
+                                        0, 0, ptr, size, L._stream(x)))
+        assert torch.equal(out, whole) or used
+        assert bool(ws.any()) == used                        # partial sums lie in it once it is used
+
+
+def test_merged_projections_beyond_short_prompts_equal_their_oracles():
+    K, M, dt = 576, 1100, torch.float16
+    cases = [Case(n, K, 128, 4, dt, seed=90 + i, bias=(i == 1), residual=16 * i) for i, n in enumerate((512, 128, 256))]
+    assert L.lib().b200lut_gemm_launch_workspace_bytes(M, 896, K, 4, 128) > 0
+    qkv = pkg.SplitQKV(*(c.module() for c in cases))
+    x = cases[0].x(M)
+    want = torch.cat([c.oracle(x) for c in cases], dim=-1)
+    for _ in range(2):                                       # Python route, native route
+        assert rel_err(qkv(x.cuda()), want) <= TOL

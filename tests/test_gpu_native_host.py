@@ -5,6 +5,7 @@ other dtype or device state), where results have to follow the module."""
 from __future__ import annotations
 
 import copy
+import random
 
 import pytest
 import torch
@@ -249,3 +250,72 @@ def test_threads_of_one_stream_do_not_mix_their_two_stream_launches():
     for t in threads:
         t.join()
     assert bad == [0] * 4
+
+
+@pytest.mark.parametrize("opts", range(len(OPTIONS)))
+@pytest.mark.parametrize("M", (1, 8, 9, 16, 17, 130))
+def test_the_native_route_serves_every_option(M, opts):
+    case = Case(256, 192, 64, 4, torch.float16, seed=70 + opts, **OPTIONS[opts])
+    mod = case.module()
+    x = case.x(M).cuda()
+    mod(x)
+    got = pkg._lib.host.linear(mod.__dict__, x, True)
+    assert got is not None and torch.equal(got, mod._forward_route(x))
+
+
+@pytest.mark.parametrize("seed", range(24))
+def test_rules_of_the_two_routes_agree(seed):
+    # the same C entries, so the same bits, wherever the native layer does not leave the call alone
+    rng = random.Random(seed)
+    bits, gs, dt = rng.choice((1, 2, 3, 4)), rng.choice((32, 64, 128, 256)), rng.choice((torch.float16, torch.bfloat16))
+    K = 64 * rng.randint(1, 9)
+    opts = dict(bias=rng.random() < 0.5, residual=rng.choice((0, 0, 8, 12, 72)), bits2=rng.choice((None, None, 1, 2, 3, 4)))
+    if rng.random() < 0.4:
+        opts.update(rotation_seed=rng.randint(0, 99), awq=rng.random() < 0.5)
+    a, b = (Case(256, K, gs, bits, dt, seed=2 * seed + i, **opts) for i in range(2))
+    qkv = pkg.SplitQKV(a.module(), b.module(), b.module())
+    mlp = pkg.FusedPalettizedMLP(a.module(), b.module(), Case(128, 256, gs, bits, dt, seed=seed, **opts).module(),
+                                 torch.nn.SiLU())
+    for M in (1, 3, 8, 9, 16, 17, 33, 130):
+        x = (0.5 * torch.randn(M, K, generator=torch.Generator().manual_seed(M))).to(dt).cuda()
+        for mod in (qkv.q_proj, qkv, mlp):
+            want = mod._forward_route(x)
+            mod(x)
+            assert torch.equal(mod(x), want), (M, type(mod).__name__)
+
+
+@pytest.mark.parametrize("kind", ("kgrouped", "two_stream"))
+def test_scratch_of_captured_graphs_and_of_many_streams(kind):
+    # two graphs of their own capture and eager calls between their replays; then more streams than the
+    # pool keeps buffers for, each used again after its buffer may have gone
+    N, K, M, dt = 512, 1024, 300, torch.float16
+    if kind == "kgrouped":
+        assert pkg._lib.lib().b200lut_gemm_workspace_bytes(M, N, K) > 0
+        lut_k = (0.02 * torch.randn(K // 128, N, 16, generator=torch.Generator().manual_seed(1))).to(dt)
+        blob = torch.randint(0, 256, (N * K // 2,), dtype=torch.uint8, generator=torch.Generator().manual_seed(2))
+        mod = pkg.KGroupedPalettizedLinear(blob, lut_k, 4, N, K).cuda()
+    else:
+        mod = Case(N, K, 128, 4, dt, seed=61, bits2=2).module()
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(3)).to(dt).cuda()
+    mod(x)
+    want = mod(x)
+    graphs, outs = [], []
+    for _ in range(2):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            outs.append(mod(x))
+        graphs.append(g)
+    for g, o in zip(graphs * 2, outs * 2):
+        g.replay()
+        assert torch.equal(mod(x), want)
+        torch.cuda.synchronize()
+        assert torch.equal(o, want)
+    streams = [torch.cuda.Stream() for _ in range(40)]
+    for _ in range(2):
+        got = []
+        for s in streams:
+            s.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(s):
+                got.append(mod(x))
+        torch.cuda.synchronize()
+        assert all(torch.equal(g, want) for g in got)
