@@ -50,8 +50,9 @@ enum {
   B200LUT_FLAG_CTA_PAIRS = 8,    /* prefill GEMM: run launches of M >= 256 rows with an even number of
                                     128-row tiles as pairs of CTAs (tcgen05 cta_group::2: one MMA
                                     covers 256 weight rows, each CTA fetches half of the activation
-                                    tile; no multicast load). Same results bit for bit, measured
-                                    slower than one CTA per tile, so it is never the default */
+                                    tile; no multicast load). With whole tiles the same results bit
+                                    for bit, measured 1.5 to 1.9 times as long as one CTA per tile, so
+                                    it is never the default */
   B200LUT_FLAG_WHOLE_TILES = 16  /* prefill GEMMs: every output (of two streams, each stream's part) is one sum
                                     over all of K: no cut of K over blocks, whatever the workspace, and one
                                     accumulator */
@@ -289,7 +290,7 @@ typedef struct b200lut_exchange {
  * segments with split = 0 (the library's policy) — the producer_blocks of an exchange whose
  * pushing launch they describe. Output pointers of the segments may be NULL here. 0 on invalid
  * arguments. The policy picks between the two decode kernels by shape and M (a launch without an
- * exchange may run the tensor-core kernel from three rows on, which has no exchange); a launch that
+ * exchange may run the tensor-core kernel from nine rows on, which has no exchange); a launch that
  * carries an input transform or a flag-less (sentinel) exchange always runs the row-range
  * kernel, so pass B200LUT_FLAG_ROWS_KERNEL here for such a launch. No counterpart in the
  * reference. */

@@ -1,8 +1,10 @@
-// LUT GEMM for batches of 3 to a few hundred rows (batched decode, short prompts) on tcgen05.
+// LUT GEMM for batches of 9 to a few hundred rows (batched decode, short prompts) on tcgen05.
 //
 // Such a launch is a stream of codes with little arithmetic per code: at 64 rows a 128 x 64 chunk of
-// 4-bit codes (4 KB of HBM, 177 cycles of an SM's share) feeds four MMAs of 128 x 64 x 16 (149
-// cycles measured, issue included). The whole-tile kernel of gemm_tc.cu took 680 to 790 cycles per
+// 4-bit codes (4 KB of HBM, 177 cycles of an SM's share; 128 wavefronts of lookups) feeds four MMAs of
+// 128 x 64 x 16, and these bound it: an MMA with its A operand in tensor memory takes about 60 cycles
+// whatever its width up to 128 columns (238 cycles per chunk at 16 to 64 tokens, 257 at 128, measured alone),
+// and the kernel takes 257 at 64 tokens. The whole-tile kernel of gemm_tc.cu took 680 to 790 cycles per
 // chunk here: eight lookup warps, each of them a serial chain of about 1450 cycles per chunk
 // (measured with the SM clock: 500 waiting for its own code load, 390 looking up and storing, 150 for
 // the next load and its cursor, the rest barriers), one tile per SM whatever the tile count.

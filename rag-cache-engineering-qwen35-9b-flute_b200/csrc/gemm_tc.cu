@@ -1155,8 +1155,9 @@ int persistent_gemm(const void* x, int64_t ldx, int M, int K, int dtype, const b
   pp.M = M; pp.K = K; pp.G = K / kChunkK;
   pp.gs = s.group_size;
   // CTA pairs (cta_group::2), on request (B200LUT_FLAG_CTA_PAIRS): the plain lookup mode only.
-  // Measured 1.47x SLOWER than one CTA per tile at every prefill shape (bit-identical results),
-  // so the library never picks it by itself.
+  // Slower than one CTA per tile at every prefill shape (with whole tiles the same bits), so the library never
+  // picks it by itself: 2048 tokens of 12288 x 4096 303 against 175 us, 24576 x 4096 550 / 375, 4096 x 12288
+  // 298 / 158, 512 tokens of 12288 x 4096 75 / 50.
   const bool pair = cta_pairs && pairs_serve(rows, M, sms) && !acc_out && !acc_in && !extra && !kgrouped;
   pp.NT = M >= kPMaxNT ? kPMaxNT : ((M + 31) / 32) * 32;
   pp.m_tiles = (M + pp.NT - 1) / pp.NT;

@@ -31,8 +31,9 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) {
 // operands from warp-uniform registers: behind this predicate the compiler knows that one thread
 // issues them, behind `lane == 0` it does not and serialises every instruction over the lanes that
 // might be active. Measured (four MMAs of 128 x N x 16 and a commit per k-block, operands resident):
-// 564 cycles per k-block at every N <= 256 with `lane == 0`; with the election 512 (the pipe) at
-// N = 256, 331 at 128, 314 at 16 to 64.
+// 564 cycles per k-block at every N <= 256 with `lane == 0`; with the election, in a ring of four operand
+// stages whose commits are waited for, 512 (the pipe) at N = 256, 385 at 192, 257 at 128 and 238 at 16 to
+// 64 (commits that pile up with nobody waiting cost more: 305 at N <= 128).
 __device__ __forceinline__ bool elect_one() {
   uint32_t on;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(on));
